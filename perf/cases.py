@@ -218,3 +218,55 @@ def run(state):
     if c["via"] == "module":
         return attention_cutlass_fp8.flash_attention_v2_cutlass(state["q"], state["k"], state["v"], c["causal"], state["scale"])
     return flash_attention_v2_cutlass(state["q"], state["k"], state["v"], c["causal"], state["scale"], v_layout=c["v"], **state["kw"])
+
+
+def _attention64(q, k, v, causal, scale, rows_at_once=2 ** 26):
+    """Softmax attention of one slice in 64 bits, q [Sq, D], k and v [Sk, D]; returns (O, log-sum-exp)."""
+    Sq, Sk = q.shape[0], k.shape[0]
+    step = max(1, rows_at_once // Sk)
+    o = torch.empty((Sq, v.shape[1]), dtype=torch.float64, device=q.device)
+    lse = torch.empty((Sq,), dtype=torch.float64, device=q.device)
+    for r in range(0, Sq, step):
+        s = (q[r:r + step] @ k.T) * scale
+        if causal:
+            n = s.shape[0]
+            s.masked_fill_(torch.arange(Sk, device=q.device) > torch.arange(r, r + n, device=q.device).unsqueeze(1), -math.inf)
+        lse[r:r + step] = torch.logsumexp(s, dim=1)
+        s -= lse[r:r + step].unsqueeze(1)
+        o[r:r + step] = s.exp_() @ v
+    return o, lse
+
+
+def _quantised(x, per_head):
+    """What quantize_e4m3 stands for, in plain torch: x * 448 / max|x| in 32 bits, rounded to e4m3; and the scale."""
+    amax = x.abs().amax(dim=(2, 3), keepdim=True).float() if per_head else x.abs().amax().float().reshape(1, 1, 1, 1)
+    return (x.float() * (448.0 / amax)).to(torch.float8_e4m3fn), (amax.double() / 448.0).reshape(-1)
+
+
+def exact(case, seed):
+    """The outputs of run() in 64 bits from the same fp8 values; the fp8 bytes of a quantisation have none of their own."""
+    c = dict(case)
+    s = prepare(c, seed)
+    if c["op"] == "quantise":
+        return None, _quantised(s["x"], c["per_head"])[1]
+    q, k, v = s["q"], s["k"], s["v"]
+    scale, transposed = s["scale"], c["op"] == "host" or c.get("v") == "transposed"
+    d = [s.get("kw", {}).get("descale_" + n) for n in "qkv"]
+    if c["op"] == "pipeline":
+        (q, dq), (k, dk), (v, dv) = (_quantised(x, c["per_head"]) for x in (q, k, v))
+        d = [dq, dk, dv]
+    device = torch.device("cuda", torch.cuda.current_device())
+    B, H, Sq, D = q.shape
+    Hk = k.shape[1]
+    o = torch.empty((B, H, Sq, D), dtype=torch.float64, device="cpu" if c["op"] == "host" else device)
+    lse = torch.empty((B, H, Sq), dtype=torch.float64, device=device)
+    at = lambda t, i: 1.0 if t is None else (t[0] if t.numel() == 1 else t[i]).double()
+    for b in range(B):
+        for h in range(H):
+            hk = h // (H // Hk)
+            q1, k1, v1 = (x.to(device).double() for x in (q[b, h], k[b, hk], v[b, hk]))
+            if transposed:
+                v1 = v1.T
+            o1, lse[b, h] = _attention64(q1 * at(d[0], b * H + h), k1 * at(d[1], b * Hk + hk), v1 * at(d[2], b * Hk + hk), c["causal"], scale)
+            o[b, h] = o1
+    return [o, lse] if c.get("lse") else [o]
