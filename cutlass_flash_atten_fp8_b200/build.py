@@ -20,7 +20,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libfa8_b200.so")
 # Digest of the sources the library was built from, written next to it: a copy of the tree keeps
 # file contents but not necessarily modification times, so staleness is decided by content.
 HASH_PATH = os.path.join(PKG_DIR, "libfa8_b200.srchash")
-SOURCES = ["fa8_fwd_sm100.cu", "fa8_quant.cu", "fa8_capi.cu"]
+SOURCES = ["fa8_fwd_sm100.cu", "fa8_decode_sm100.cu", "fa8_quant.cu", "fa8_capi.cu"]
 HEADERS = ["fa8_kernel.h", "ptx_sm100.cuh", os.path.join(REPO_DIR, "include", "fa8_b200.h")]
 
 

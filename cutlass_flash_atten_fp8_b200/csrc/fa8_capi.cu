@@ -215,6 +215,9 @@ int fa8_supported(int32_t seqlen_k, int32_t head_dim, int32_t v_layout) {
 // head dim of the kernel that serves `head_dim` (the next of 64, 128, 256)
 static int kernel_head_dim(int32_t head_dim) { return head_dim <= 64 ? 64 : (head_dim <= 128 ? 128 : 256); }
 
+// Most query rows (heads of a group times query positions) that go to the decode kernel.
+constexpr int64_t kDecodeRows = 64;
+
 int fa8_work_plan(int32_t slices, int32_t seqlen, int32_t seqlen_k, int32_t head_dim, int32_t is_causal,
                   int32_t sm_count, int32_t plan[4]) {
   if (!plan || slices <= 0 || seqlen <= 0 || seqlen_k < 0 || sm_count <= 0) return FA8_ERR_BAD_ARG;
@@ -249,7 +252,7 @@ int fa8_fwd(const fa8_fwd_params* p, void* cuda_stream) {
   const int32_t seqlen_k = p->seqlen_k > 0 ? p->seqlen_k : p->seqlen;
   int sup = fa8_supported(seqlen_k, p->head_dim, p->v_layout);
   if (sup != FA8_OK) return sup;
-  const int64_t bh = static_cast<int64_t>(p->batch) * p->heads;
+  const int64_t bh_q = static_cast<int64_t>(p->batch) * p->heads;
   const int32_t heads_kv = p->heads_kv > 0 ? p->heads_kv : p->heads;
   if (heads_kv > p->heads || p->heads % heads_kv != 0) return FA8_ERR_BAD_ARG;
   const int64_t bh_kv = static_cast<int64_t>(p->batch) * heads_kv;
@@ -264,7 +267,50 @@ int fa8_fwd(const fa8_fwd_params* p, void* cuda_stream) {
     set_detail("an earlier launch on this device reported an expired wait", buf);
     return FA8_ERR_DEVICE_TIMEOUT;
   }
-  const uint64_t S = static_cast<uint64_t>(p->seqlen), D = static_cast<uint64_t>(p->head_dim);
+  // one work item per 128 query rows is the finest plan the launcher can choose
+  if (bh_q * ((static_cast<int64_t>(p->seqlen) + 127) / 128) > 0x7fffffff) return FA8_ERR_UNSUPPORTED;
+  // Without a causal mask the query heads that share a key/value head see the same keys, and their
+  // rows are contiguous in Q, O and the log-sum-exp: a group of heads is one slice of
+  // group * seqlen rows.
+  const int32_t group = p->heads / heads_kv;
+  const int64_t rows = static_cast<int64_t>(group) * p->seqlen;
+  int* const status = p->status_word ? p->status_word : (dstate ? dstate->dev_word : nullptr);
+  int* const host_status = dstate ? dstate->host_flag_dev : nullptr;
+  if (!p->is_causal && p->v_layout == FA8_V_NATURAL && rows <= kDecodeRows && bh_kv * kDecodeRows <= 0x7fffffff) {
+    fa8::DecodeArgs da{};
+    da.q = static_cast<const uint8_t*>(p->q);
+    da.k = static_cast<const uint8_t*>(p->k);
+    da.v = static_cast<const uint8_t*>(p->v);
+    da.o = static_cast<__half*>(p->o);
+    da.lse = p->softmax_lse;
+    da.n_slices = static_cast<int>(bh_kv);
+    da.rows = static_cast<int>(rows);
+    da.seqlen_q = p->seqlen;
+    da.seqlen_k = seqlen_k;
+    da.head_dim = p->head_dim;
+    da.group = group;
+    da.scale_log2 = p->softmax_scale * 1.4426950408889634f;
+    da.o_scale = p->o_scale;
+    da.descale_q = p->descale_q;
+    da.descale_k = p->descale_k;
+    da.descale_v = p->descale_v;
+    da.descale_per_head = p->descale_per_head != 0;
+    da.status = status;
+    da.host_status = host_status;
+    const cudaError_t e = fa8::launch_decode(da, p->fp8_format == FA8_FP8_E5M2, stream);
+    if (e != cudaSuccess) {
+      set_detail("kernel launch", cudaGetErrorString(e));
+      return FA8_ERR_CUDA;
+    }
+    return FA8_OK;
+  }
+  // Elsewhere a folded group saves padding when it needs fewer 128-row tiles (4 heads of 65
+  // rows: 3 tiles instead of 4).
+  const bool fold = !p->is_causal && group > 1 && rows <= 0x7fffffff - 256 &&
+                    (rows + 127) / 128 < static_cast<int64_t>(group) * ((static_cast<int64_t>(p->seqlen) + 127) / 128);
+  const int64_t bh = fold ? bh_kv : bh_q;
+  const uint64_t S = fold ? static_cast<uint64_t>(rows) : static_cast<uint64_t>(p->seqlen);
+  const uint64_t D = static_cast<uint64_t>(p->head_dim);
   const uint64_t Sk = static_cast<uint64_t>(seqlen_k);
   // The kernel is built for head dims 64, 128 and 256 (the reference's switch has eight
   // buckets, csrc/static_switch.h:50-77).  The others run on the next one up: the tensor maps
@@ -316,24 +362,23 @@ int fa8_fwd(const fa8_fwd_params* p, void* cuda_stream) {
 
   fa8::KernelArgs args;
   args.o = static_cast<__half*>(p->o);
-  args.seqlen = p->seqlen;
+  args.seqlen = static_cast<int>(S);
   args.seqlen_k = seqlen_k;
   args.head_dim = p->head_dim;
   args.scale_log2 = p->softmax_scale * 1.4426950408889634f;
   args.o_scale = p->o_scale;
-  args.status = p->status_word ? p->status_word : (dstate ? dstate->dev_word : nullptr);
-  args.host_status = dstate ? dstate->host_flag_dev : nullptr;
+  args.status = status;
+  args.host_status = host_status;
   args.lse = p->softmax_lse;
   args.descale_q = p->descale_q;
   args.descale_k = p->descale_k;
   args.descale_v = p->descale_v;
   args.descale_per_head = p->descale_per_head != 0;
-  args.heads = p->heads;
+  args.q_fold = fold ? group : 1;
+  args.heads = fold ? heads_kv : p->heads;
   args.heads_kv = heads_kv;
   args.softmax_scale = p->softmax_scale;
   args.timeout_ns = 2000000000ull;
-  // one work item per 128 query rows is the finest plan the launcher can choose
-  if (bh * ((static_cast<int64_t>(p->seqlen) + 127) / 128) > 0x7fffffff) return FA8_ERR_UNSUPPORTED;
   args.n_slices = static_cast<int>(bh);
   cudaError_t e = fa8::launch_fwd(static_cast<int>(d_box), p->is_causal != 0, p->v_layout == FA8_V_NATURAL,
                                   p->fp8_format == FA8_FP8_E5M2, tq, tk, tv, to, args, stream);

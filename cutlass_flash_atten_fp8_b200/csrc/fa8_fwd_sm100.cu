@@ -907,7 +907,10 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             const int kv_bh = b_idx * args.heads_kv + (w.bh - b_idx * args.heads) / (args.heads / args.heads_kv);
             qk_descale = 1.f;
             o_scale = args.o_scale;
-            if (args.descale_q != nullptr) qk_descale *= __ldg(args.descale_q + w.bh);
+            // (rows past the last one take the last one's scale: their results are dropped)
+            if (args.descale_q != nullptr)
+              qk_descale *= __ldg(args.descale_q + (args.q_fold == 1 ? w.bh : w.bh * args.q_fold + min(q_row, seqlen - 1) /
+                                                                                  (seqlen / args.q_fold)));
             if (args.descale_k != nullptr) qk_descale *= __ldg(args.descale_k + kv_bh);
             if (args.descale_v != nullptr) o_scale *= __ldg(args.descale_v + kv_bh);
             c = args.scale_log2 * qk_descale;

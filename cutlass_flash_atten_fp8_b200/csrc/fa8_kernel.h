@@ -31,6 +31,8 @@ struct KernelArgs {
   const float* descale_k;
   const float* descale_v;
   int descale_per_head;           // the three are arrays: [batch*heads] for Q, [batch*heads_kv] for K, V
+  int q_fold;                     // heads of the caller's Q that are rows of one slice here (1 = none): row r of
+                                  // slice s has the scale descale_q[s * q_fold + r / (seqlen / q_fold)]
   float* lse;                     // optional [batch*heads, seqlen] fp32: log-sum-exp of the scaled scores
   float softmax_scale;            // as given by the caller (natural-log units, for lse)
   int* status;                    // device word; non-zero after a bounded wait expired (later CTAs then return at once)
@@ -48,6 +50,39 @@ struct KernelArgs {
 cudaError_t launch_fwd(int head_dim, bool causal, bool v_natural, bool e5m2, const CUtensorMap& tq,
                        const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& to, const KernelArgs& args,
                        cudaStream_t stream);
+
+// Few query rows against many keys without a causal mask (fa8_decode_sm100.cu): the query heads
+// that share a key/value head are rows of one tile.
+struct DecodeArgs {
+  const uint8_t* q;               // [n_slices, rows, head_dim]
+  const uint8_t* k;               // [n_slices, seqlen_k, head_dim]
+  const uint8_t* v;               // the same (natural layout)
+  __half* o;                      // [n_slices, rows, head_dim]
+  float* lse;                     // optional [n_slices, rows]
+  int n_slices;                   // batch * heads_kv
+  int rows;                       // group * seqlen_q
+  int seqlen_q;                   // query positions: row r belongs to head r / seqlen_q of its group
+  int seqlen_k;
+  int head_dim;                   // a multiple of 32 up to 256
+  int group;                      // query heads per key/value head
+  float scale_log2;               // as in KernelArgs
+  float o_scale;
+  const float* descale_q;
+  const float* descale_k;
+  const float* descale_v;
+  int descale_per_head;
+  int* status;                    // non-zero at launch: nothing is computed or written
+  int* host_status;
+  // Filled in by launch_decode: blocks of rows a slice is cut into, CTAs (one cluster) its keys
+  // are split over.
+  int row_blocks;
+  int n_split;
+};
+cudaError_t launch_decode(const DecodeArgs& a, bool e5m2, cudaStream_t stream);
+
+// How launch_decode splits the keys of `items` (slices times row blocks): CTAs per cluster, and
+// the warps of each in *warps.  Host arithmetic only.
+int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int* warps);
 
 // The work plan launch_fwd would choose on a GPU of `sms` SMs: fills rows_per_item, n_pairs,
 // fold and n_units of `a` from its seqlen, seqlen_k and n_slices.  Host arithmetic only.

@@ -1,0 +1,90 @@
+"""Few query rows against many keys (no causal mask, V as [keys, head_dim]): the decode kernel, and
+the folding of query heads that share a key/value head into one slice.
+
+Against the kernel model (the same rounding of P to fp8, starting maximum over the first 64 keys) the
+difference is the order of fp32 sums and, now and then, a P on the other side of a rounding step: 2e-3 as
+for the prefill kernel.  Against the fp32 oracle it is the rounding of P: 3e-2 (e5m2 6e-2)."""
+import math
+
+import pytest
+import torch
+
+from cutlass_flash_atten_fp8_b200 import check_status, flash_attention_v2_cutlass
+from oracle.attention_oracle import attention_quantised_p, error_metrics
+
+pytestmark = pytest.mark.gpu
+KERNEL_MODEL = dict(block_n=64, lazy=True, lazy_limit=448.0, lazy_rows=32)
+
+
+def rand8(*shape, seed, dtype=torch.float8_e4m3fn, scale=1.0):
+    return (torch.randn(*shape, generator=torch.Generator().manual_seed(seed)) * scale).to(dtype)
+
+
+def call(q, k, v, scale, **kw):
+    d = torch.device("cuda", 0)
+    n = q.numel()
+    guard = torch.full((n + 64,), float("nan"), dtype=torch.float16, device=d)
+    out, lse = flash_attention_v2_cutlass(q.to(d), k.to(d), v.to(d), False, scale, v_layout="natural", return_lse=True,
+                                          out=guard[:n].view(q.shape), **kw)
+    check_status(d)
+    assert bool(torch.isnan(guard[n:]).all())
+    return out.float().cpu(), lse.cpu()
+
+
+def reference(q, k, v, scale):
+    g = q.shape[1] // k.shape[1]
+    s = q.float() @ k.float().repeat_interleave(g, 1).transpose(2, 3) * scale
+    return torch.softmax(s, -1) @ v.float().repeat_interleave(g, 1), torch.logsumexp(s, -1)
+
+
+# one key, less than the first 64, not a multiple of a 32-key step, one step more than a split of two to
+# eight CTAs of four warps; 1, 7, 8, 9, 16, 17, 64 and 65 rows (the last one past the decode kernel)
+@pytest.mark.parametrize("H,Hk,Sq,Sk,D", [
+    (2, 2, 1, 1, 32), (2, 1, 1, 33, 64), (4, 2, 1, 64, 128), (7, 1, 1, 65, 128), (8, 1, 1, 1000, 256), (3, 1, 3, 777, 96),
+    (2, 1, 8, 4097, 64), (17, 1, 1, 2049, 160), (16, 2, 8, 1056, 128), (5, 1, 13, 513, 192), (8, 1, 2, 288, 224)])
+@pytest.mark.parametrize("dtype", [torch.float8_e4m3fn, torch.float8_e5m2])
+def test_against_the_oracles(H, Hk, Sq, Sk, D, dtype):
+    q, k, v = (rand8(2, h, s, D, seed=Sk + i, dtype=dtype) for i, (h, s) in enumerate([(H, Sq), (Hk, Sk), (Hk, Sk)]))
+    scale = 1 / math.sqrt(D)
+    e4m3 = dtype == torch.float8_e4m3fn
+    out, lse = call(q, k, v, scale)
+    g = H // Hk
+    model = attention_quantised_p(q, k.float().repeat_interleave(g, 1).to(dtype), v.float().repeat_interleave(g, 1).to(dtype), False,
+                                  scale, p_format="e4m3" if e4m3 else "e5m2", **KERNEL_MODEL)
+    assert error_metrics(out, model)["rel_l2"] <= 2e-3
+    ref, ref_lse = reference(q, k, v, scale)
+    assert float((lse - ref_lse).abs().max()) <= 1e-5 * float(ref_lse.abs().max()) + 1e-5
+    # scores of a few units: the maximum over the first 64 keys is outgrown by later ones
+    q6 = (q.float() * 6).to(dtype)
+    out, lse = call(q6, k, v, scale)
+    ref, ref_lse = reference(q6, k, v, scale)
+    assert error_metrics(out, ref)["rel_l2"] <= (3e-2 if e4m3 else 6e-2)
+    assert float((lse - ref_lse).abs().max()) <= 1e-5 * float(ref_lse.abs().max()) + 1e-5
+
+
+@pytest.mark.parametrize("Sq,Sk", [(1, 700), (3, 700), (100, 300)])
+def test_scales_per_head_follow_the_heads_of_a_group(Sq, Sk):
+    H, Hk, D = 6, 2, 64
+    q, k, v = rand8(2, H, Sq, D, seed=1), rand8(2, Hk, Sk, D, seed=2), rand8(2, Hk, Sk, D, seed=3)
+    d = torch.device("cuda", 0)
+    dq, dk, dv = (0.5 + torch.rand(2 * n, generator=torch.Generator().manual_seed(n)) for n in (H, Hk, Hk))
+    out, lse = call(q, k, v, 0.125, descale_q=dq.to(d), descale_k=dk.to(d), descale_v=dv.to(d))
+    ref, ref_lse = reference(q.float() * dq.view(2, H, 1, 1), k.float() * dk.view(2, Hk, 1, 1), v.float() * dv.view(2, Hk, 1, 1), 0.125)
+    assert error_metrics(out, ref)["rel_l2"] <= 3e-2
+    assert float((lse - ref_lse).abs().max()) <= 1e-4
+
+
+def test_a_stale_status_word_leaves_the_output_alone():
+    d = torch.device("cuda", 0)
+    q, k, v = (rand8(1, 2, s, 64, seed=s).to(d) for s in (1, 512, 512))
+    word = torch.ones(1, dtype=torch.int32, device=d)
+    out = torch.full((1, 2, 1, 64), 7.0, dtype=torch.float16, device=d)
+    flash_attention_v2_cutlass(q, k, v, False, 0.125, v_layout="natural", out=out, _status=word)
+    torch.cuda.synchronize()
+    assert bool((out == 7.0).all())
+    with pytest.raises(RuntimeError):              # the host has been told; the next call reports it
+        flash_attention_v2_cutlass(q, k, v, False, 0.125, v_layout="natural", out=out, _status=word)
+    word.zero_()
+    flash_attention_v2_cutlass(q, k, v, False, 0.125, v_layout="natural", out=out, _status=word)
+    check_status(d, word=word)
+    assert not bool((out == 7.0).any())
