@@ -215,9 +215,6 @@ int fa8_supported(int32_t seqlen_k, int32_t head_dim, int32_t v_layout) {
 // head dim of the kernel that serves `head_dim` (the next of 64, 128, 256)
 static int kernel_head_dim(int32_t head_dim) { return head_dim <= 64 ? 64 : (head_dim <= 128 ? 128 : 256); }
 
-// Most query rows (heads of a group times query positions) that go to the decode kernel.
-constexpr int64_t kDecodeRows = 64;
-
 int fa8_work_plan(int32_t slices, int32_t seqlen, int32_t seqlen_k, int32_t head_dim, int32_t is_causal,
                   int32_t sm_count, int32_t plan[4]) {
   if (!plan || slices <= 0 || seqlen <= 0 || seqlen_k < 0 || sm_count <= 0) return FA8_ERR_BAD_ARG;
@@ -276,7 +273,13 @@ int fa8_fwd(const fa8_fwd_params* p, void* cuda_stream) {
   const int64_t rows = static_cast<int64_t>(group) * p->seqlen;
   int* const status = p->status_word ? p->status_word : (dstate ? dstate->dev_word : nullptr);
   int* const host_status = dstate ? dstate->host_flag_dev : nullptr;
-  if (!p->is_causal && p->v_layout == FA8_V_NATURAL && rows <= kDecodeRows && bh_kv * kDecodeRows <= 0x7fffffff) {
+  cudaError_t se = cudaSuccess;
+  const int sms = fa8::current_sm_count(&se);
+  if (sms <= 0) {
+    set_detail("SM count", cudaGetErrorString(se));
+    return FA8_ERR_CUDA;
+  }
+  if (!p->is_causal && p->v_layout == FA8_V_NATURAL && fa8::decode_takes(bh_kv, rows, seqlen_k, p->head_dim, sms)) {
     fa8::DecodeArgs da{};
     da.q = static_cast<const uint8_t*>(p->q);
     da.k = static_cast<const uint8_t*>(p->k);
@@ -297,7 +300,7 @@ int fa8_fwd(const fa8_fwd_params* p, void* cuda_stream) {
     da.descale_per_head = p->descale_per_head != 0;
     da.status = status;
     da.host_status = host_status;
-    const cudaError_t e = fa8::launch_decode(da, p->fp8_format == FA8_FP8_E5M2, stream);
+    const cudaError_t e = fa8::launch_decode(da, p->fp8_format == FA8_FP8_E5M2, sms, stream);
     if (e != cudaSuccess) {
       set_detail("kernel launch", cudaGetErrorString(e));
       return FA8_ERR_CUDA;

@@ -11,9 +11,9 @@
 //   * a slice's keys are split over a thread-block cluster and over the warps of each of its
 //     CTAs; the partial sums are put together through distributed shared memory, so the split
 //     needs no workspace and no second launch;
-//   * a warp streams 32 keys at a time from global memory straight into the registers of
-//     mma.m16n8k32 operands (all loads are 8 or 16 bytes a thread, whole 32-byte sectors),
-//     the next keys' loads in flight while the current ones are worked on.  There is no
+//   * a warp streams 32 keys at a time from global memory straight into registers, in the order
+//     in which mma.m16n8k16 wants its operands (all loads are 8 or 16 bytes a thread, whole
+//     32-byte sectors), the next keys' loads in flight while the current ones are worked on.  There is no
 //     shared-memory staging, hence no barrier and no wait in the loop.  tcgen05 would want 128
 //     rows (or 128 lanes of keys and a transposed P through shared memory) for what is 24 small
 //     products per 8 KB read.
@@ -21,10 +21,10 @@
 // Operand layouts.  S = Q K^T with the query rows as M (16, eight of them padding when RB = 1)
 // and eight keys as N; the k index of the instruction may be permuted as long as both operands
 // agree, so thread (g, t) = (lane / 4, lane % 4) takes bytes 16 t .. 16 t + 15 of every 64 of a
-// row: one 16-byte load holds its words for two k-steps.  O^T = V^T P^T with 16 output columns as
-// M, the rows as N and 32 keys as k: a thread's P values of four score tiles are the k words of
-// the B operand as they stand, and its A words are four keys of one column, byte-transposed in
-// registers (2 PRMT per word) from rows of V.
+// row: each of the four words of a 16-byte load, widened to fp16, is its part of one k-step.
+// O^T = V^T P^T with 16 output columns as M, the rows as N and 16 keys as k: a thread's P values of
+// two score tiles are its part of the B operand as they stand, and its part of the A operand is
+// two columns of four keys, paired up by byte permutations of rows of V.
 //
 // Numerics are those of the prefill kernel: P = 2^(c s - c m) in fp32, rounded to fp8 after the
 // fp32 row sum, with m the exact row maximum over the first 64 keys of the slice (every warp of
@@ -35,7 +35,6 @@
 
 #include <atomic>
 #include <cstdint>
-#include <cstdlib>
 
 #include "fa8_kernel.h"
 #include "ptx_sm100.cuh"
@@ -50,34 +49,38 @@ constexpr int kStepKeys = 32;          // keys of one warp step = k of one PV in
 constexpr int kFirstKeys = 64;         // keys the starting maximum is taken over
 constexpr float kRaiseAbove = 448.f;   // largest e4m3 value
 
+// Every fp8 value is an fp16 value too, so a product of widened operands with an fp32 sum is the fp8
+// product.  The instruction's own fp8 form is carried out in fp16 as well on this architecture, but
+// widens both operands again for every product; widening each K and V word once by hand takes
+// about half as many
+// instructions (652 per warp step before, counted by ncu; 57 us before, 51 now at batch 16, 8 key/value
+// heads, 8192 keys, head dim 128).
+__device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// Four fp8 -> two pairs of fp16, ascending.
 template <bool kE5M2>
-__device__ __forceinline__ void mma_fp8(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void widen4(uint32_t w, uint32_t& lo, uint32_t& hi) {
   if (kE5M2) {
-    asm("mma.sync.aligned.m16n8k32.row.col.f32.e5m2.e5m2.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\t"
+        "cvt.rn.f16x2.e5m2x2 %0, l;\n\tcvt.rn.f16x2.e5m2x2 %1, h;\n\t}" : "=r"(lo), "=r"(hi) : "r"(w));
   } else {
-    asm("mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+    asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\t"
+        "cvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}" : "=r"(lo), "=r"(hi) : "r"(w));
   }
 }
 
+// Two fp32 rounded to fp8, as a pair of fp16.
 template <bool kE5M2>
-__device__ __forceinline__ uint32_t pack4(float a, float b, float c, float d) {
+__device__ __forceinline__ uint32_t round2(float a, float b) {
   uint32_t r;
   if (kE5M2) {
-    asm("{\n\t.reg .b16 lo, hi;\n\t"
-        "cvt.rn.satfinite.e5m2x2.f32 lo, %2, %1;\n\t"
-        "cvt.rn.satfinite.e5m2x2.f32 hi, %4, %3;\n\t"
-        "mov.b32 %0, {lo, hi};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
+    asm("{\n\t.reg .b16 x;\n\tcvt.rn.satfinite.e5m2x2.f32 x, %2, %1;\n\tcvt.rn.f16x2.e5m2x2 %0, x;\n\t}" : "=r"(r) : "f"(a), "f"(b));
   } else {
-    asm("{\n\t.reg .b16 lo, hi;\n\t"
-        "cvt.rn.satfinite.e4m3x2.f32 lo, %2, %1;\n\t"
-        "cvt.rn.satfinite.e4m3x2.f32 hi, %4, %3;\n\t"
-        "mov.b32 %0, {lo, hi};\n\t}"
-        : "=r"(r) : "f"(a), "f"(b), "f"(c), "f"(d));
+    asm("{\n\t.reg .b16 x;\n\tcvt.rn.satfinite.e4m3x2.f32 x, %2, %1;\n\tcvt.rn.f16x2.e4m3x2 %0, x;\n\t}" : "=r"(r) : "f"(a), "f"(b));
   }
   return r;
 }
@@ -94,23 +97,13 @@ __device__ __forceinline__ uint2 ld_stream8(const uint8_t* p) {
   return v;
 }
 
-// 4 x 4 byte transpose: out[i] = byte i of x0, x1, x2, x3.
-__device__ __forceinline__ void transpose4(uint32_t x0, uint32_t x1, uint32_t x2, uint32_t x3, uint32_t (&out)[4]) {
-  const uint32_t lo01 = __byte_perm(x0, x1, 0x5140), lo23 = __byte_perm(x2, x3, 0x5140);
-  const uint32_t hi01 = __byte_perm(x0, x1, 0x7362), hi23 = __byte_perm(x2, x3, 0x7362);
-  out[0] = __byte_perm(lo01, lo23, 0x5410);
-  out[1] = __byte_perm(lo01, lo23, 0x7632);
-  out[2] = __byte_perm(hi01, hi23, 0x5410);
-  out[3] = __byte_perm(hi01, hi23, 0x7632);
-}
-
 // Head dims up to W run in the instance built for W; bytes past head_dim are zeros in registers.
 // RB: blocks of eight query rows a CTA works on (16 rows need a second PV product per column
 // block; at W = 256 their accumulators do not fit the registers).
 template <int W, int RB>
 struct DCfg {
   static constexpr int kChunks = W / 64;                 // 64-byte pieces of a K row
-  static constexpr int kSteps = W / 32;                  // k-steps of Q K^T
+  static constexpr int kSteps = W / 16;                  // k-steps of Q K^T
   static constexpr int kVWords = W == 64 ? 2 : 4;        // V words of a thread per key and column block
   static constexpr int kVBlocks = W == 256 ? 2 : 1;      // column blocks of 128
   static constexpr int kTilesPerBlock = 2 * kVWords;     // PV products (16 columns each) per column block
@@ -125,7 +118,8 @@ struct DCfg {
   }
 };
 
-template <int W, int RB, bool kE5M2>
+// kExact: head_dim is W.
+template <int W, int RB, bool kE5M2, bool kExact>
 __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_kernel(const DecodeArgs a) {
   using C = DCfg<W, RB>;
   extern __shared__ __align__(16) float smem[];
@@ -142,7 +136,7 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
   const int work = blockIdx.x / n_split;
   const int slice = work / a.row_blocks;
   const int row0 = (work - slice * a.row_blocks) * C::kRows;
-  const int D = a.head_dim, Sk = a.seqlen_k;
+  const int D = kExact ? W : a.head_dim, Sk = a.seqlen_k;
   // An earlier launch's expired wait is still in the status word: leave O alone, tell the host
   // (as the prefill kernel does).  The barriers below are passed all the same.
   const bool stale = __any_sync(0xffffffffu, a.status != nullptr && *reinterpret_cast<volatile int*>(a.status) != 0);
@@ -165,7 +159,7 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
 #pragma unroll
     for (int c = 0; c < C::kChunks; ++c) {
       r[c] = make_uint4(0u, 0u, 0u, 0u);
-      if (64 * c + k_col < D) r[c] = ld_stream16(p + 64 * c);
+      if (kExact || 64 * c + k_col < D) r[c] = ld_stream16(p + 64 * c);
     }
   };
   auto load_v = [&](uint32_t (&r)[8][C::kVWords], int key0, int blk) {
@@ -176,7 +170,7 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
       const uint8_t* p = vp + static_cast<size_t>(min(key, Sk - 1)) * D + col;
 #pragma unroll
       for (int w = 0; w < C::kVWords; ++w) r[i][w] = 0u;
-      if (col < D) {
+      if (kExact || col < D) {
         if constexpr (C::kVWords == 2) {
           const uint2 x = ld_stream8(p);
           r[i][0] = x.x; r[i][1] = x.y;
@@ -189,25 +183,33 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
   };
 
   // Q rows as A operands; rows past the last one are zeros.
-  uint32_t qa[C::kSteps][4];
+  uint32_t qa[C::kSteps][RB][2];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < RB; ++h) {
     const int row = row0 + g + 8 * h;
     const uint8_t* p = a.q + (static_cast<size_t>(slice) * a.rows + row) * D + k_col;
 #pragma unroll
     for (int c = 0; c < C::kChunks; ++c) {
       uint4 x = make_uint4(0u, 0u, 0u, 0u);
-      if (h < RB && row < a.rows && 64 * c + k_col < D) x = __ldg(reinterpret_cast<const uint4*>(p + 64 * c));
-      qa[2 * c][h] = x.x;     qa[2 * c][2 + h] = x.y;
-      qa[2 * c + 1][h] = x.z; qa[2 * c + 1][2 + h] = x.w;
+      if (row < a.rows && 64 * c + k_col < D) x = __ldg(reinterpret_cast<const uint4*>(p + 64 * c));
+      widen4<kE5M2>(x.x, qa[4 * c][h][0], qa[4 * c][h][1]);
+      widen4<kE5M2>(x.y, qa[4 * c + 1][h][0], qa[4 * c + 1][h][1]);
+      widen4<kE5M2>(x.z, qa[4 * c + 2][h][0], qa[4 * c + 2][h][1]);
+      widen4<kE5M2>(x.w, qa[4 * c + 3][h][0], qa[4 * c + 3][h][1]);
     }
   }
   auto scores = [&](const uint4 (&kr)[C::kChunks], float (&s)[4]) {
     s[0] = s[1] = s[2] = s[3] = 0.f;
 #pragma unroll
     for (int c = 0; c < C::kChunks; ++c) {
-      mma_fp8<kE5M2>(s, qa[2 * c], kr[c].x, kr[c].y);
-      mma_fp8<kE5M2>(s, qa[2 * c + 1], kr[c].z, kr[c].w);
+      const uint32_t w[4] = {kr[c].x, kr[c].y, kr[c].z, kr[c].w};
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        uint32_t b0, b1;
+        widen4<kE5M2>(w[u], b0, b1);
+        const auto& qw = qa[4 * c + u];
+        mma_f16(s, qw[0][0], RB == 2 ? qw[RB - 1][0] : 0u, qw[0][1], RB == 2 ? qw[RB - 1][1] : 0u, b0, b1);
+      }
     }
   };
 
@@ -335,25 +337,32 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
         }
         exponentials();
       }
-      uint32_t pb[RB][2];
+      uint32_t pb[RB][4];                                 // one word per score tile
 #pragma unroll
       for (int h = 0; h < RB; ++h) {
         l_row[h] += sum[h];
-        pb[h][0] = pack4<kE5M2>(p[h][0], p[h][1], p[h][2], p[h][3]);
-        pb[h][1] = pack4<kE5M2>(p[h][4], p[h][5], p[h][6], p[h][7]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) pb[h][j] = round2<kE5M2>(p[h][2 * j], p[h][2 * j + 1]);
       }
 #pragma unroll
       for (int blk = 0; blk < C::kVBlocks; ++blk) {
 #pragma unroll
         for (int w = 0; w < C::kVWords; ++w) {
-          uint32_t x[4], y[4];
-          transpose4(vr[0][w], vr[1][w], vr[2][w], vr[3][w], x);
-          transpose4(vr[4][w], vr[5][w], vr[6][w], vr[7][w], y);
-          const uint32_t a0[4] = {x[0], x[1], y[0], y[1]}, a1[4] = {x[2], x[3], y[2], y[3]};
 #pragma unroll
-          for (int h = 0; h < RB; ++h) {
-            mma_fp8<kE5M2>(o[blk * C::kTilesPerBlock + 2 * w][h], a0, pb[h][0], pb[h][1]);
-            mma_fp8<kE5M2>(o[blk * C::kTilesPerBlock + 2 * w + 1][h], a1, pb[h][0], pb[h][1]);
+          for (int u = 0; u < 2; ++u) {                   // 16 keys each
+            // bytes of two keys side by side, two columns a word
+            const uint32_t* x = &vr[4 * u][w];
+            constexpr int kKey = C::kVWords;              // words from one key to the next
+            uint32_t a[4][2];
+            widen4<kE5M2>(__byte_perm(x[0], x[kKey], 0x5140), a[0][0], a[1][0]);
+            widen4<kE5M2>(__byte_perm(x[2 * kKey], x[3 * kKey], 0x5140), a[0][1], a[1][1]);
+            widen4<kE5M2>(__byte_perm(x[0], x[kKey], 0x7362), a[2][0], a[3][0]);
+            widen4<kE5M2>(__byte_perm(x[2 * kKey], x[3 * kKey], 0x7362), a[2][1], a[3][1]);
+#pragma unroll
+            for (int h = 0; h < RB; ++h) {
+              mma_f16(o[blk * C::kTilesPerBlock + 2 * w][h], a[0][0], a[1][0], a[0][1], a[1][1], pb[h][2 * u], pb[h][2 * u + 1]);
+              mma_f16(o[blk * C::kTilesPerBlock + 2 * w + 1][h], a[2][0], a[3][0], a[2][1], a[3][1], pb[h][2 * u], pb[h][2 * u + 1]);
+            }
           }
         }
         if (blk + 1 < C::kVBlocks) load_v(vr, key0, blk + 1);
@@ -437,10 +446,10 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
   if (n_split > 1) cluster.sync();                         // no CTA leaves while its shared memory is read
 }
 
-template <int W, int RB, bool kE5M2>
-cudaError_t launch_decode_one(DecodeArgs a, int sms, cudaStream_t stream) {
+template <int W, int RB, bool kE5M2, bool kExact>
+cudaError_t launch_decode_inst(DecodeArgs a, int sms, cudaStream_t stream) {
   using C = DCfg<W, RB>;
-  auto kernel = &fa8_decode_kernel<W, RB, kE5M2>;
+  auto kernel = &fa8_decode_kernel<W, RB, kE5M2, kExact>;
   static std::atomic<uint64_t> opted_in{0};                // one bit per device: kernel attributes set
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -469,6 +478,12 @@ cudaError_t launch_decode_one(DecodeArgs a, int sms, cudaStream_t stream) {
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
+template <int W, int RB, bool kE5M2>
+cudaError_t launch_decode_one(const DecodeArgs& a, int sms, cudaStream_t stream) {
+  return a.head_dim == W ? launch_decode_inst<W, RB, kE5M2, true>(a, sms, stream)
+                         : launch_decode_inst<W, RB, kE5M2, false>(a, sms, stream);
+}
+
 template <bool kE5M2>
 cudaError_t launch_decode_fmt(const DecodeArgs& a, int sms, cudaStream_t stream) {
   if (a.head_dim <= 64)
@@ -480,14 +495,10 @@ cudaError_t launch_decode_fmt(const DecodeArgs& a, int sms, cudaStream_t stream)
 
 }  // namespace
 
-#ifndef FA8_DEC_TUNE
-#define FA8_DEC_TUNE 0      // 1: measurement build, split and warps from the environment
-#endif
-
 // As many warps as one wave of the GPU holds, every one with at least a step of its own; among
 // equals the smallest CTAs.  A second, partly filled wave costs more than the warps it adds
-// (batch 16, 8 key/value heads, 8192 keys, head dim 128: 57 us with three CTAs of four warps per
-// slice, 384 of the 444 that fit; 70 with two, 77 with four).
+// (batch 16, 8 key/value heads, 8192 keys, head dim 128, an earlier form of the kernel: 57 us with
+// three CTAs of four warps per slice, 384 of the 444 that fit; 70 with two, 77 with four).
 int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int* warps) {
   const int steps = (seqlen_k + kStepKeys - 1) / kStepKeys;
   int best_split = 1, best_warps = 4;
@@ -503,27 +514,44 @@ int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int* warps
     if (nw > 4 && items * split > static_cast<int64_t>(sms) * (max_warps / nw)) continue;
     if (busy > best) { best = busy; best_split = static_cast<int>(split); best_warps = nw; }
   }
-#if FA8_DEC_TUNE
-  if (const char* s = getenv("FA8_DEC_SPLIT")) best_split = atoi(s);
-  if (const char* s = getenv("FA8_DEC_WARPS")) best_warps = atoi(s);
-#endif
   *warps = best_warps;
   return best_split;
 }
 
-cudaError_t launch_decode(const DecodeArgs& a, bool e5m2, cudaStream_t stream) {
+// Up to kDecodeRowsMax rows may come here.  A single block of rows always does: 5.2 TB/s of K and V
+// (78 % of a copy) against a step of 0.41 us per 64 keys (0.65 at head dim 256) and slice of the
+// prefill kernel.  Several blocks each read K and V (from L2, at the same rate per SM), so they
+// do when the prefill kernel would leave SMs idle - it does not split a slice's keys.  Measured,
+// head dim 128: 8 slices of 56 rows, 16384 keys of head dim 64: 18 us here, 105 there; 128 slices of
+// 48 rows, 4096 keys: 98 us here, 33 there.
+bool decode_takes(int64_t slices, int64_t rows, int seqlen_k, int head_dim, int sms) {
+  const int width = head_dim <= 64 ? 64 : (head_dim <= 128 ? 128 : 256);
+  const int64_t block = width == 256 ? 8 : 16;
+  const int64_t row_blocks = (rows + block - 1) / block;
+  if (rows > kDecodeRowsMax || slices * row_blocks * 8 > 0x7fffffff) return false;
+  if (row_blocks == 1) return true;
+  const double keys = seqlen_k;
+  const double here = static_cast<double>(row_blocks) * slices * keys * 2.0 * width / 5.2e6;                  // us
+  const double there = static_cast<double>((slices + sms - 1) / sms) * (keys / 64.0 * (width == 256 ? 0.65 : 0.41) + 3.0);
+  return here < there;
+}
+
+int current_sm_count(cudaError_t* e) {
   static std::atomic<int> sm_count[64];
   int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+  *e = cudaGetDevice(&dev);
+  if (*e != cudaSuccess) return 0;
   const bool cached = dev >= 0 && dev < 64;
   int sms = cached ? sm_count[dev].load(std::memory_order_acquire) : 0;
   if (sms == 0) {
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    if (sms <= 0) return cudaErrorInvalidDevice;
+    *e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (*e != cudaSuccess) return 0;
     if (cached) sm_count[dev].store(sms, std::memory_order_release);
   }
+  return sms;
+}
+
+cudaError_t launch_decode(const DecodeArgs& a, bool e5m2, int sms, cudaStream_t stream) {
   return e5m2 ? launch_decode_fmt<true>(a, sms, stream) : launch_decode_fmt<false>(a, sms, stream);
 }
 

@@ -78,7 +78,12 @@ struct DecodeArgs {
   int row_blocks;
   int n_split;
 };
-cudaError_t launch_decode(const DecodeArgs& a, bool e5m2, cudaStream_t stream);
+cudaError_t launch_decode(const DecodeArgs& a, bool e5m2, int sms, cudaStream_t stream);
+constexpr int64_t kDecodeRowsMax = 63;
+// Whether a launch of `slices` slices of `rows` rows each is one for launch_decode.
+bool decode_takes(int64_t slices, int64_t rows, int seqlen_k, int head_dim, int sms);
+// SMs of the current device (kept per device); 0 and *e on failure.
+int current_sm_count(cudaError_t* e);
 
 // How launch_decode splits the keys of `items` (slices times row blocks): CTAs per cluster, and
 // the warps of each in *warps.  Host arithmetic only.

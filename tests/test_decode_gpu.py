@@ -1,7 +1,7 @@
 """Few query rows against many keys (no causal mask, V as [keys, head_dim]): the decode kernel, and
 the folding of query heads that share a key/value head into one slice.
 
-Against the kernel model (the same rounding of P to fp8, starting maximum over the first 64 keys) the
+Against a model of it (the same rounding of P to fp8, starting maximum over the first 64 keys) the
 difference is the order of fp32 sums and, now and then, a P on the other side of a rounding step: 2e-3 as
 for the prefill kernel.  Against the fp32 oracle it is the rounding of P: 3e-2 (e5m2 6e-2)."""
 import math
@@ -10,10 +10,9 @@ import pytest
 import torch
 
 from cutlass_flash_atten_fp8_b200 import check_status, flash_attention_v2_cutlass
-from oracle.attention_oracle import attention_quantised_p, error_metrics
+from oracle.attention_oracle import error_metrics
 
 pytestmark = pytest.mark.gpu
-KERNEL_MODEL = dict(block_n=64, lazy=True, lazy_limit=448.0, lazy_rows=32)
 
 
 def rand8(*shape, seed, dtype=torch.float8_e4m3fn, scale=1.0):
@@ -37,6 +36,15 @@ def reference(q, k, v, scale):
     return torch.softmax(s, -1) @ v.float().repeat_interleave(g, 1), torch.logsumexp(s, -1)
 
 
+def rounded_p(q, k, v, scale, dtype):
+    """P relative to the maximum over the first 64 keys, rounded to fp8 for P V but not for the row sum."""
+    g = q.shape[1] // k.shape[1]
+    s = q.float() @ k.float().repeat_interleave(g, 1).transpose(2, 3) * scale
+    p = torch.exp(s - s[..., :64].amax(-1, keepdim=True))
+    assert float(p.max()) <= 448.0                  # the maximum is not raised
+    return p.to(dtype).float() @ v.float().repeat_interleave(g, 1) / p.sum(-1, keepdim=True)
+
+
 # one key, less than the first 64, not a multiple of a 32-key step, one step more than a split of two to
 # eight CTAs of four warps; 1, 7, 8, 9, 16, 17, 64 and 65 rows (the last one past the decode kernel)
 @pytest.mark.parametrize("H,Hk,Sq,Sk,D", [
@@ -48,10 +56,7 @@ def test_against_the_oracles(H, Hk, Sq, Sk, D, dtype):
     scale = 1 / math.sqrt(D)
     e4m3 = dtype == torch.float8_e4m3fn
     out, lse = call(q, k, v, scale)
-    g = H // Hk
-    model = attention_quantised_p(q, k.float().repeat_interleave(g, 1).to(dtype), v.float().repeat_interleave(g, 1).to(dtype), False,
-                                  scale, p_format="e4m3" if e4m3 else "e5m2", **KERNEL_MODEL)
-    assert error_metrics(out, model)["rel_l2"] <= 2e-3
+    assert error_metrics(out, rounded_p(q, k, v, scale, dtype))["rel_l2"] <= 2e-3
     ref, ref_lse = reference(q, k, v, scale)
     assert float((lse - ref_lse).abs().max()) <= 1e-5 * float(ref_lse.abs().max()) + 1e-5
     # scores of a few units: the maximum over the first 64 keys is outgrown by later ones
