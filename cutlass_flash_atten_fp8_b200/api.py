@@ -10,13 +10,31 @@ its C ABI.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 from typing import List, Optional
 
 import torch
 
-from . import _lib
+from . import _lib, build
 
 _status_words = {}
+_native_module = None        # the compiled module once asked for, False where it has not been built
+
+
+def _native():
+    """The compiled torch module (csrc/torch_binding.cpp), whose _forward and _quantize take the calls
+    that nothing is wrong with.  False where it is missing or older than its source: every call is
+    then made from here, through ctypes."""
+    global _native_module
+    if _native_module is None:
+        _lib.load()              # raises if the library itself is missing or stale
+        module = False
+        if not build.binding_is_stale():
+            spec = importlib.util.spec_from_file_location(build.BINDING_NAME, build.binding_path())
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+        _native_module = module
+    return _native_module
 
 
 def _check_input(x: torch.Tensor, name: str) -> None:
@@ -31,7 +49,10 @@ def status_word(device: torch.device) -> torch.Tensor:
     """The int32 device word kernels on `device` report an expired wait into."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
     if idx not in _status_words:
-        _status_words[idx] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
+        word = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
+        _status_words[idx] = word            # held here for good: the compiled module keeps its address
+        if _native():
+            _native()._set_status_word(idx, word.data_ptr())
     return _status_words[idx]
 
 
@@ -80,6 +101,17 @@ def flash_attention_v2_cutlass(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     return_lse=True appends the fp32 [batch, heads, seqlen] log-sum-exp of the scaled
     scores (the reference reserves softmax_lse_ptr for it, csrc/flash.h:56, unused).
     """
+    native = _native()
+    if native and (v_layout == "transposed" or v_layout == "natural"):
+        try:
+            done = native._forward(q, k, v, is_causal, softmax_scale, v_layout == "natural", o_scale, out, return_lse,
+                                   descale_q, descale_k, descale_v, _status)
+        except TypeError:        # arguments of other types: the checks below say which, or convert them
+            done = None
+        if type(done) is list:
+            return done
+        if done is not None:
+            raise RuntimeError(_lib.error_message(done))
     lib = _lib.load()
     _check_input(q, "q")
     _check_input(k, "k")
@@ -150,6 +182,16 @@ def quantize_e4m3(x: torch.Tensor, per_head: bool = False):
     one-element fp32 tensor; with per_head=True x is [batch, heads, ...] and every (batch,
     head) slice gets its own scale: descale is [batch*heads].  Stream-ordered, two HBM-bound
     kernels; stands where the reference's callers cast with torch (test.py:20-22, 68-70)."""
+    native = _native()
+    if native:
+        try:
+            done = native._quantize(x, bool(per_head))
+        except TypeError:
+            done = None
+        if type(done) is tuple:
+            return done
+        if done is not None:
+            raise RuntimeError(_lib.error_message(done))
     lib = _lib.load()
     _check_input(x, "x")
     if x.dtype not in (torch.float16, torch.bfloat16):
