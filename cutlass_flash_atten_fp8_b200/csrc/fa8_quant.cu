@@ -1,20 +1,30 @@
-// Per-tensor amax quantisation fp16/bf16 -> e4m3: the step before the attention path in
-// the reference's own pipeline (test.py:12-23 casts with torch, test.py:68-70), here as two
-// HBM-bound kernels so that a caller can go from half-precision Q/K/V to the FP8 operator
-// without leaving the stream.
+// Amax quantisation fp16/bf16 -> e4m3: the step before the attention path in the reference's own
+// pipeline (test.py:12-23 casts with torch, test.py:68-70), here so that a caller can go from
+// half-precision Q/K/V to the FP8 operator without leaving the stream.
 //
-//   pass 1  amax = max |x|             reads 2N bytes, one atomicMax per CTA into *amax
-//   pass 2  y = e4m3(x * 448 / amax)   reads 2N bytes, writes N bytes; round-to-nearest-even,
-//           descale = amax / 448       saturating (cvt.rn.satfinite.e4m3x2.f32)
+//   amax = max |x|,  y = e4m3(x * 448 / amax) round-to-nearest-even, saturating,  descale = amax / 448
 //
-// Both use 16-byte loads, a grid of a few CTAs per SM and grid-stride loops.  amax and descale
-// are caller-provided device floats (outputs); nothing else is written.  With n_seg > 1 the
-// tensor is n_seg equal, contiguous segments (one per head, say), each with its own amax and
-// descale: blockIdx.y picks the segment.
+// of one tensor, or (n_seg > 1) of n_seg equal, contiguous segments of it (one per head, say), each
+// with its own amax and descale.  amax and descale are caller-provided device floats (outputs);
+// nothing else is written.  Bound by memory: 2 bytes read and 1 written per element would do, but
+// every element depends on the maximum of all.  Two forms:
+//
+//   segment_kernel   a segment per thread-block cluster, one launch: the maximum is exchanged through
+//                    distributed shared memory, what a thread read first stays in its registers
+//                    and the rest is read again while it is still in L2, so HBM sees 3 bytes per
+//                    element.
+//   whole_kernel     one long segment, one cooperative launch of the whole GPU with a grid barrier
+//                    between the passes: the first 48 MB (registers and shared memory of 148 SMs)
+//                    are read once, the rest again, last to first.
+//   amax_kernel +    several long segments, or a very long one: two passes over the tensor (5 bytes per element), the
+//   cast_kernel      second last to first.  amax is cleared before by a memset and accumulated
+//                    with atomicMax.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 #include "fa8_kernel.h"
@@ -24,7 +34,19 @@ namespace fa8 {
 
 namespace {
 
-constexpr int kQuantThreads = 256;
+namespace cg = cooperative_groups;
+
+// 16-byte vectors at the end of the first pass that are meant to stay in L2 for the second: the ones
+// before them are read as streamed data, first to be replaced.  96 MB of a 256 MB tensor: 107.2 us; 64 MB
+// 108.3, none 112.8 (the second pass forwards, neither marked as streamed: 116.4).
+constexpr int64_t kKeep = 96ll << 16;
+// Longest lone segment of whole_kernel: 128 MB 50.5 us against 55.6 in two passes, 256 MB 111 against 107.
+constexpr int64_t kWholeMaxVec = 192ll << 16;
+constexpr int kQuantThreads = 256;     // of the two-pass kernels
+constexpr int kSegThreads = 512;       // most threads of a segment_kernel CTA
+constexpr int kHold = 8;               // 16-byte vectors of a thread that stay in registers between the passes
+constexpr int kStage = 12;             // whole_kernel: further ones that stay in shared memory
+constexpr int kStageBytes = kStage * kSegThreads * 16;
 
 template <bool kBf16>
 __device__ __forceinline__ float2 unpack_pair(uint32_t w) {
@@ -36,104 +58,336 @@ __device__ __forceinline__ float2 unpack_pair(uint32_t w) {
   return __half22float2(h);
 }
 
+// Running maximum of |x| over 16-byte vectors, kept as packed pairs of the source type (the
+// maximum of a set of its numbers is one of them, so nothing is rounded).  max drops NaN inputs,
+// so a NaN does not reach amax (it still casts to the fp8 NaN); an infinite input makes amax
+// infinite, the scale 448/inf = 0 and every finite output 0 (inf * 0 = NaN for the infinite ones):
+// inputs are expected to be finite.
 template <bool kBf16>
-__global__ void __launch_bounds__(kQuantThreads) amax_kernel(const uint4* __restrict__ x, int64_t n_vec,
+struct AbsMax {
+  uint32_t m[2] = {0u, 0u};
+  __device__ __forceinline__ void pair(int k, uint32_t w) {
+    w &= 0x7fff7fffu;
+    if (kBf16) asm("max.bf16x2 %0, %0, %1;" : "+r"(m[k]) : "r"(w));
+    else asm("max.f16x2 %0, %0, %1;" : "+r"(m[k]) : "r"(w));
+  }
+  __device__ __forceinline__ void take(const uint4& v) {
+    pair(0, v.x); pair(1, v.y); pair(0, v.z); pair(1, v.w);
+  }
+  __device__ __forceinline__ float value() const {
+    const float2 a = unpack_pair<kBf16>(m[0]), b = unpack_pair<kBf16>(m[1]);
+    return fmaxf(fmaxf(a.x, a.y), fmaxf(b.x, b.y));
+  }
+};
+
+// Maximum over the CTA, valid in every thread.
+__device__ __forceinline__ float cta_max(float m) {
+  __shared__ float part[kSegThreads / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
+  __syncthreads();
+  for (int w = 0; w < (blockDim.x >> 5); ++w) m = fmaxf(m, part[w]);
+  return m;
+}
+
+template <bool kBf16>
+__device__ __forceinline__ uint2 cast8(const uint4& v, float scale) {
+  const float2 f0 = unpack_pair<kBf16>(v.x), f1 = unpack_pair<kBf16>(v.y);
+  const float2 f2 = unpack_pair<kBf16>(v.z), f3 = unpack_pair<kBf16>(v.w);
+  uint2 o;
+  o.x = cvt_e4m3x2(f0.x * scale, f0.y * scale) | (cvt_e4m3x2(f1.x * scale, f1.y * scale) << 16);
+  o.y = cvt_e4m3x2(f2.x * scale, f2.y * scale) | (cvt_e4m3x2(f3.x * scale, f3.y * scale) << 16);
+  return o;
+}
+__device__ __forceinline__ float scale_of(float amax) { return amax > 0.f ? 448.f / amax : 1.f; }
+__device__ __forceinline__ float descale_of(float amax) { return amax > 0.f ? amax / 448.f : 1.f; }
+
+// n_vec = 16-byte vectors of a segment; the n_tail elements behind them exist for a lone segment only.
+template <bool kBf16>
+__global__ void __launch_bounds__(kSegThreads, 2) segment_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
+                                                                 int64_t n_vec, const uint16_t* __restrict__ tail_in,
+                                                                 uint8_t* __restrict__ tail_out, int n_tail, int csize,
+                                                                 float* __restrict__ amax, float* __restrict__ descale) {
+  __shared__ float peers[8];
+  const int seg = blockIdx.x / csize, rank = blockIdx.x - seg * csize;
+  x += seg * n_vec;
+  y += seg * n_vec;
+  const int64_t stride = static_cast<int64_t>(csize) * blockDim.x;
+  const int64_t i0 = static_cast<int64_t>(rank) * blockDim.x + threadIdx.x;
+  uint4 hold[kHold];
+  AbsMax<kBf16> mx;
+  // A CTA may be written to by its peers once all of them run: told now, waited for below.
+  if (csize > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+#pragma unroll
+  for (int u = 0; u < kHold; ++u) {
+    const int64_t i = i0 + u * stride;
+    hold[u] = i < n_vec ? x[i] : make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int u = 0; u < kHold; ++u) mx.take(hold[u]);
+  const int64_t first = i0 + kHold * stride;               // what does not fit the registers
+#pragma unroll 4
+  for (int64_t i = first; i < n_vec; i += stride) mx.take(x[i]);
+  float tail = 0.f;
+  const bool has_tail = rank == 0 && threadIdx.x < n_tail;
+  if (has_tail) {
+    tail = unpack_pair<kBf16>(tail_in[threadIdx.x]).x;
+    mx.pair(0, tail_in[threadIdx.x]);
+  }
+  float a = cta_max(mx.value());
+  if (csize > 1) {
+    // Every CTA leaves its maximum with all of them: after the one barrier only local memory is read.
+    cg::cluster_group cluster = cg::this_cluster();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (threadIdx.x < csize) *cluster.map_shared_rank(&peers[rank], static_cast<int>(threadIdx.x)) = a;
+    cluster.sync();
+    for (int p = 0; p < csize; ++p) a = fmaxf(a, peers[p]);
+  }
+  if (rank == 0 && threadIdx.x == 0) {
+    amax[seg] = a;
+    if (descale != nullptr) descale[seg] = descale_of(a);
+  }
+  const float scale = scale_of(a);
+  if (first < n_vec) {
+    // last to first: what was read last is the nearest
+#pragma unroll 4
+    for (int64_t i = first + (n_vec - 1 - first) / stride * stride; i >= first; i -= stride)
+      y[i] = cast8<kBf16>(x[i], scale);
+  }
+#pragma unroll
+  for (int u = 0; u < kHold; ++u) {
+    const int64_t i = i0 + u * stride;
+    if (i < n_vec) y[i] = cast8<kBf16>(hold[u], scale);
+  }
+  if (has_tail) tail_out[threadIdx.x] = static_cast<uint8_t>(cvt_e4m3x2(tail * scale, 0.f) & 0xffu);
+}
+
+template <bool kBf16>
+__global__ void __launch_bounds__(kSegThreads, 2) whole_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
+                                                               int64_t n_vec, const uint16_t* __restrict__ tail_in,
+                                                               uint8_t* __restrict__ tail_out, int n_tail,
+                                                               float* amax, float* __restrict__ descale) {
+  extern __shared__ uint4 stage[];                         // [kStage][thread]: every thread reads its own
+  cg::grid_group grid = cg::this_grid();
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *amax = 0.f;
+  uint4 hold[kHold];
+  AbsMax<kBf16> mx;
+#pragma unroll
+  for (int u = 0; u < kHold; ++u) {
+    const int64_t i = i0 + u * stride;
+    hold[u] = i < n_vec ? x[i] : make_uint4(0u, 0u, 0u, 0u);
+  }
+  grid.sync();                                             // amax is cleared; the loads are on their way
+#pragma unroll
+  for (int u = 0; u < kHold; ++u) mx.take(hold[u]);
+  const int64_t staged = i0 + kHold * stride, first = staged + kStage * stride;
+  if (staged < n_vec) {
+#pragma unroll
+    for (int u = 0; u < kStage; ++u) {
+      const int64_t i = staged + u * stride;
+      if (i < n_vec) {
+        const uint4 v = x[i];
+        stage[u * kSegThreads + threadIdx.x] = v;
+        mx.take(v);
+      }
+    }
+  }
+  const int64_t keep_from = n_vec - kKeep;
+  int64_t j = first;
+#pragma unroll 4
+  for (; j < keep_from; j += stride) mx.take(__ldcs(x + j));
+#pragma unroll 4
+  for (; j < n_vec; j += stride) mx.take(x[j]);
+  float tail = 0.f;
+  const bool has_tail = blockIdx.x == 0 && threadIdx.x < n_tail;
+  if (has_tail) {
+    tail = unpack_pair<kBf16>(tail_in[threadIdx.x]).x;
+    mx.pair(0, tail_in[threadIdx.x]);
+  }
+  const float m = cta_max(mx.value());
+  // non-negative floats order like their bit patterns
+  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m));
+  grid.sync();
+  const float a = *reinterpret_cast<volatile float*>(amax);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && descale != nullptr) *descale = descale_of(a);
+  const float scale = scale_of(a);
+  if (first < n_vec) {
+#pragma unroll 4
+    for (int64_t i = first + (n_vec - 1 - first) / stride * stride; i >= first; i -= stride)
+      __stcs(y + i, cast8<kBf16>(__ldcs(x + i), scale));
+  }
+  if (staged < n_vec) {
+#pragma unroll
+    for (int u = kStage - 1; u >= 0; --u) {
+      const int64_t i = staged + u * stride;
+      if (i < n_vec) y[i] = cast8<kBf16>(stage[u * kSegThreads + threadIdx.x], scale);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kHold; ++u) {
+    const int64_t i = i0 + u * stride;
+    if (i < n_vec) y[i] = cast8<kBf16>(hold[u], scale);
+  }
+  if (has_tail) tail_out[threadIdx.x] = static_cast<uint8_t>(cvt_e4m3x2(tail * scale, 0.f) & 0xffu);
+}
+
+template <bool kBf16>
+__global__ void __launch_bounds__(kQuantThreads, 8) amax_kernel(const uint4* __restrict__ x, int64_t n_vec,
                                                             const uint16_t* __restrict__ tail, int n_tail,
                                                             float* __restrict__ amax) {
   x += blockIdx.y * n_vec;
   amax += blockIdx.y;
-  float m = 0.f;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint4 v = x[i];
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const float2 f = unpack_pair<kBf16>(w[k]);
-      m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x < n_tail) {
-    const uint32_t w = tail[threadIdx.x];
-    m = fmaxf(m, fabsf(unpack_pair<kBf16>(w).x));
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ float part[kQuantThreads / 32];
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < kQuantThreads / 32 ? part[threadIdx.x] : 0.f;
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    // Non-negative floats order like their bit patterns.  fmaxf drops NaN inputs, so a NaN does
-    // not reach amax (it still casts to the fp8 NaN in pass 2); an infinite input makes amax
-    // infinite, the scale 448/inf = 0 and every finite output 0 (inf * 0 = NaN for the infinite
-    // ones): inputs are expected to be finite.
-    if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m));
-  }
+  AbsMax<kBf16> mx;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  const int64_t keep_from = n_vec - kKeep / gridDim.y;
+  int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+#pragma unroll 4
+  for (; i < keep_from; i += stride) mx.take(__ldcs(x + i));
+#pragma unroll 4
+  for (; i < n_vec; i += stride) mx.take(x[i]);
+  if (blockIdx.x == 0 && threadIdx.x < n_tail) mx.pair(0, tail[threadIdx.x]);
+  const float m = cta_max(mx.value());
+  // non-negative floats order like their bit patterns
+  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m));
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kQuantThreads) cast_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
+__global__ void __launch_bounds__(kQuantThreads, 8) cast_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
                                                             int64_t n_vec, const uint16_t* __restrict__ tail_in,
                                                             uint8_t* __restrict__ tail_out, int n_tail,
                                                             const float* __restrict__ amax,
                                                             float* __restrict__ descale) {
   x += blockIdx.y * n_vec;
   y += blockIdx.y * n_vec;
-  amax += blockIdx.y;
-  if (descale != nullptr) descale += blockIdx.y;
-  const float a = *amax;
-  const float scale = a > 0.f ? 448.f / a : 1.f;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && descale != nullptr) *descale = a > 0.f ? a / 448.f : 1.f;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_vec;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const uint4 v = x[i];
-    const float2 f0 = unpack_pair<kBf16>(v.x), f1 = unpack_pair<kBf16>(v.y);
-    const float2 f2 = unpack_pair<kBf16>(v.z), f3 = unpack_pair<kBf16>(v.w);
-    uint2 o;
-    o.x = cvt_e4m3x2(f0.x * scale, f0.y * scale) | (cvt_e4m3x2(f1.x * scale, f1.y * scale) << 16);
-    o.y = cvt_e4m3x2(f2.x * scale, f2.y * scale) | (cvt_e4m3x2(f3.x * scale, f3.y * scale) << 16);
-    y[i] = o;
-  }
+  const float a = amax[blockIdx.y];
+  const float scale = scale_of(a);
+  if (blockIdx.x == 0 && threadIdx.x == 0 && descale != nullptr) descale[blockIdx.y] = descale_of(a);
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+#pragma unroll 4
+  for (int64_t i = n_vec - 1 - (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x); i >= 0; i -= stride)
+    __stcs(y + i, cast8<kBf16>(__ldcs(x + i), scale));
   if (blockIdx.x == 0 && threadIdx.x < n_tail) {
     const float f = unpack_pair<kBf16>(tail_in[threadIdx.x]).x * scale;
     tail_out[threadIdx.x] = static_cast<uint8_t>(cvt_e4m3x2(f, 0.f) & 0xffu);
   }
 }
 
+template <bool kBf16>
+cudaError_t launch_segments(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
+                            int n_seg, float* amax, float* descale, cudaStream_t stream) {
+  // as many CTAs as it takes to hold the segment in registers, at most a cluster of eight
+  const int threads = n_vec <= 1024 ? 128 : kSegThreads;
+  int csize = 1;
+  while (csize < 8 && n_vec > static_cast<int64_t>(csize) * threads * kHold) csize *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(n_seg) * csize, 1, 1);
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = csize;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = csize > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, &segment_kernel<kBf16>, x, y, n_vec, tail_in, tail_out, n_tail, csize, amax, descale);
+}
+
+// CTAs of whole_kernel that the device holds at once (0 = cannot be launched), kept per device.
+template <bool kBf16>
+int whole_capacity(int dev, int sms) {
+  static std::atomic<int> known[64];                       // 1 + the capacity
+  const bool cached = dev >= 0 && dev < 64;
+  int c = cached ? known[dev].load(std::memory_order_acquire) : 0;
+  if (c == 0) {
+    int coop = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
+        cudaFuncSetAttribute(&whole_kernel<kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, &whole_kernel<kBf16>, kSegThreads, kStageBytes) != cudaSuccess) {
+      cudaGetLastError();
+      per_sm = 0;
+    }
+    c = 1 + per_sm * sms;
+    if (cached) known[dev].store(c, std::memory_order_release);
+  }
+  return c - 1;
+}
+
+template <bool kBf16>
+cudaError_t launch_whole(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
+                         float* amax, float* descale, int capacity, cudaStream_t stream) {
+  const int64_t want = (n_vec + kSegThreads * kHold - 1) / (kSegThreads * kHold);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(want < capacity ? want : capacity), 1, 1);
+  cfg.blockDim = dim3(kSegThreads, 1, 1);
+  cfg.dynamicSmemBytes = want <= capacity ? 0 : kStageBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, &whole_kernel<kBf16>, x, y, n_vec, tail_in, tail_out, n_tail, amax, descale);
+}
+
+template <bool kBf16>
+cudaError_t launch_two_pass(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
+                            int n_seg, float* amax, float* descale, int sms, cudaStream_t stream) {
+  const int64_t want = (n_vec + kQuantThreads - 1) / kQuantThreads;
+  const int64_t cap = (8ll * sms + n_seg - 1) / n_seg;      // about eight CTAs per SM in all
+  const dim3 grid(static_cast<unsigned>(want < 1 ? 1 : (want > cap ? cap : want)), static_cast<unsigned>(n_seg), 1);
+  cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(float) * n_seg, stream);
+  if (e != cudaSuccess) return e;
+  amax_kernel<kBf16><<<grid, kQuantThreads, 0, stream>>>(x, n_vec, tail_in, n_tail, amax);
+  cast_kernel<kBf16><<<grid, kQuantThreads, 0, stream>>>(x, y, n_vec, tail_in, tail_out, n_tail, amax, descale);
+  return cudaGetLastError();
+}
+
+// Which form (us, fp16, measured on segments of the given size):
+//   up to 512 KB a cluster holds a segment in registers: 16 x 128 KB 8.3 two-pass, 4.3 by cluster;
+//   up to 1.5 MB the second half is read again from L2, worth it when there are enough clusters to
+//   fill the GPU: 128 x 1 MB 64 -> 55, 32 x 1 MB 20.2 -> 15.7, 16 x 1 MB 14.5 -> 12.5, but 4 x 2 MB 12.4 -> 17;
+//   one long segment: 2 MB 8.4 -> 6.0, 8 MB 11.9 -> 7.2, 32 MB 19.6 -> 16.5, 128 MB 64 -> 50.5;
+//   anything longer: two passes.
+template <bool kBf16>
+cudaError_t launch_any(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
+                       int n_seg, float* amax, float* descale, cudaStream_t stream) {
+  if (n_vec <= 32 * 1024 || (n_vec <= 96 * 1024 && n_seg >= 12))
+    return launch_segments<kBf16>(x, y, n_vec, tail_in, tail_out, n_tail, n_seg, amax, descale, stream);
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const int sms = current_sm_count(&e);
+  if (sms <= 0) return e;
+  if (n_seg == 1 && n_vec <= kWholeMaxVec) {
+    const int capacity = whole_capacity<kBf16>(dev, sms);
+    if (capacity > 0) {
+      e = launch_whole<kBf16>(x, y, n_vec, tail_in, tail_out, n_tail, amax, descale, capacity, stream);
+      // fewer SMs than the device has may be open to this process: then two passes
+      if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+      cudaGetLastError();
+    }
+  }
+  return launch_two_pass<kBf16>(x, y, n_vec, tail_in, tail_out, n_tail, n_seg, amax, descale, sms, stream);
+}
+
 }  // namespace
 
 cudaError_t launch_quantize(const void* src, bool bf16, void* dst, int64_t n, int n_seg, float* amax,
                             float* descale, cudaStream_t stream) {
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
   // n = elements per segment; segments other than a lone one are whole 16-byte vectors
   const int64_t n_vec = n / 8;
   const int n_tail = static_cast<int>(n - n_vec * 8);
   if (n_seg < 1 || n_seg > 65535 || (n_seg > 1 && n_tail != 0)) return cudaErrorInvalidValue;
-  const int64_t want = (n_vec + kQuantThreads - 1) / kQuantThreads;
-  const int64_t cap = (8ll * sms + n_seg - 1) / n_seg;      // about eight CTAs per SM in all
-  const dim3 grid(static_cast<unsigned>(want < 1 ? 1 : (want > cap ? cap : want)), static_cast<unsigned>(n_seg), 1);
   const uint4* x = static_cast<const uint4*>(src);
+  uint2* y = static_cast<uint2*>(dst);
   const uint16_t* tail_in = static_cast<const uint16_t*>(src) + n_vec * 8;
   uint8_t* tail_out = static_cast<uint8_t*>(dst) + n_vec * 8;
-  e = cudaMemsetAsync(amax, 0, sizeof(float) * n_seg, stream);
-  if (e != cudaSuccess) return e;
-  if (bf16) {
-    amax_kernel<true><<<grid, kQuantThreads, 0, stream>>>(x, n_vec, tail_in, n_tail, amax);
-    cast_kernel<true><<<grid, kQuantThreads, 0, stream>>>(x, static_cast<uint2*>(dst), n_vec, tail_in, tail_out,
-                                                          n_tail, amax, descale);
-  } else {
-    amax_kernel<false><<<grid, kQuantThreads, 0, stream>>>(x, n_vec, tail_in, n_tail, amax);
-    cast_kernel<false><<<grid, kQuantThreads, 0, stream>>>(x, static_cast<uint2*>(dst), n_vec, tail_in, tail_out,
-                                                           n_tail, amax, descale);
-  }
-  return cudaGetLastError();
+  return bf16 ? launch_any<true>(x, y, n_vec, tail_in, tail_out, n_tail, n_seg, amax, descale, stream)
+              : launch_any<false>(x, y, n_vec, tail_in, tail_out, n_tail, n_seg, amax, descale, stream);
 }
 
 }  // namespace fa8
