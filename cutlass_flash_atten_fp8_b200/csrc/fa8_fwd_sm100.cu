@@ -120,13 +120,21 @@ struct Cfg {
   //   head_dim  64: 3 x 64 + 64  = 256;  with three buffers the score of a warp's next sub-block
   //                 is computed while the warp still works on the current one
   //   head_dim 128: 2 x 64 + 128 = 256
-  //   head_dim 256: 2 x 64 + 256 = 384 of 512 (four buffers fit; measured no faster)
-#ifndef FA8_D256_NB
-#define FA8_D256_NB 2
-#endif
-  static constexpr int kSBuf = (D == 64) ? 3 : (D == 128 ? 2 : FA8_D256_NB);
+  //   head_dim 256: 4 x 64 + 256 = 512
+  static constexpr int kSBuf = (D == 64) ? 3 : (D == 128 ? 2 : 4);
   static constexpr uint32_t kTileCols = kTmemCols / kTiles;     // tile i starts at column i * kTileCols
   static constexpr uint32_t kOCol = kSubN * kSBuf;              // O follows the tile's score buffers
+  // kWide: the scores of a whole K tile come from one product, M128 N128, into two buffers side by
+  // side.  At head_dim 256 the tensor side is what limits (taking the exponentials out changes
+  // nothing, halving the k-steps of QK 14 %), and QK is bound by operand reads from shared memory: at
+  // N64 32 KB of Q for 16 KB of K, 768 cycles per 128 keys, at N128 512.  With four buffers the scores
+  // run up to two K tiles ahead of PV, so K is loaded one tile further ahead of V (K0 K1 V0 K2 V1 ...):
+  // a ring of four tiles, held up by V, could not have the next K in time (408 us that way).
+  // B2 H16 S4096: 301 us with two buffers at N64, 291 with four, 262 at N128; causal 197, 188, 175.
+  // (Measured and not kept: P in columns of its own, stored before its turn, 295; tiles of 64
+  // keys, 291; PV at N256, no change.)
+  static constexpr bool kWide = D == 256;
+  static_assert(!kWide || (kTiles == 1 && kSBuf == 4), "the order of loads and products is written for one tile and four buffers");
   static_assert(kOCol + D <= kTileCols, "tensor-memory budget");
   static_assert(4 * kW * kTiles <= 16, "sixteen softmax warps");
   static constexpr int kSlots = (D == 128) ? 8 : (D == 64 ? 16 : 4);   // ring slots, one K or V tile each
@@ -617,8 +625,13 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // Grouped-query attention: query head h of a batch entry reads K/V head h / group.
             const int b_idx = w.bh / args.heads;
             const int kv_bh = b_idx * args.heads_kv + (w.bh - b_idx * args.heads) / (args.heads / args.heads_kv);
+            if constexpr (C::kWide) load_kv(&tm_k, true, 0, 0, kv_bh);
             for (int j = 0; j < w.nb && ok; ++j) {
-              load_kv(&tm_k, true, 0, j * kBlockN, kv_bh);
+              if constexpr (C::kWide) {
+                if (j + 1 < w.nb) load_kv(&tm_k, true, 0, (j + 1) * kBlockN, kv_bh);
+              } else {
+                load_kv(&tm_k, true, 0, j * kBlockN, kv_bh);
+              }
               if (kVNatural) load_kv(&tm_v, true, 0, j * kBlockN, kv_bh);    // [keys, head_dim] rows
               else load_kv(&tm_v, false, j * kBlockN, 0, kv_bh);             // [head_dim, keys] rows
             }
@@ -656,7 +669,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       if (elect_one()) {
         const int i = warp - kMmaWarp0;
         constexpr uint32_t kFmt = kE5M2 ? 1u : 0u;
-        constexpr uint32_t kIdescQK = umma_idesc(kTileM, kSubN, kFmt);
+        constexpr uint32_t kIdescQK = umma_idesc(kTileM, C::kWide ? kBlockN : kSubN, kFmt);
         // V in its natural [keys, head_dim] layout is an MN-major B operand (bit 16).
         constexpr uint32_t kIdescPV = umma_idesc(kTileM, C::kBlkD, kFmt) | (kVNatural ? (1u << 16) : 0u);
         constexpr uint32_t kBlk16 = C::kBlkBytes / 16;       // one column block in descriptor address units
@@ -796,11 +809,21 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 // that PV has just read.  K_t (load ld + 2t) serves the QKs of sub-blocks 2t and
                 // 2t + 1, V_t (load ld + 2t + 1) their PVs; each goes back after its last reader.
                 constexpr int kNB = C::kSBuf;
+                //
+                // kWide: one product per K tile, of both its sub-blocks, into two buffers side by side:
+                // sub-blocks s and s + 1 after PV(s - 3).  Loads K_0, K_1, V_0, K_2, V_1, ...
                 auto qk_step = [&](int s, int b) -> bool {          // false when a wait ran out
-                  const uint32_t lk = ld + 2u * static_cast<uint32_t>(s >> 1);
+                  if (C::kWide && (s & 1)) return true;
+                  const uint32_t lk = C::kWide ? ld + static_cast<uint32_t>(max(s - 1, 0)) : ld + 2u * static_cast<uint32_t>(s >> 1);
                   if ((s & 1) == 0 && !kv_wait(lk)) return false;
                   issue_qk(t_tile + b * kSubN, q_lo, kv_lo(lk) + ((s & 1) ? kKHalf : 0u));
                   tc_commit(bar_s_full(i, b));
+                  if (C::kWide) {
+                    if (s + 1 < nsb) tc_commit(bar_s_full(i, b + 1));
+                    if (s + 2 >= nsb) tc_commit(b_qe);
+                    kv_release(lk);
+                    return true;
+                  }
                   if (s == nsb - 1) tc_commit(b_qe);
                   if ((s & 1) || s == nsb - 1) kv_release(lk);
                   return true;
@@ -811,7 +834,8 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 for (int sq = 0; sq < kNB && sq < nsb && ok; ++sq) ok = qk_step(sq, sq);
                 int b = 0;
                 for (int sb = 0; sb < nsb && ok; ++sb) {
-                  const uint32_t lv = ld + 2u * static_cast<uint32_t>(sb >> 1) + 1u;
+                  const uint32_t lv = C::kWide ? ld + static_cast<uint32_t>(min(2 * (sb >> 1) + 2, 2 * w.nb - 1))
+                                               : ld + 2u * static_cast<uint32_t>(sb >> 1) + 1u;
                   if ((sb & 1) == 0) ok = kv_wait(lv);
                   if (ok) ok = wait_bounded(wctx, bar_p_full(i, b), (pp >> b) & 1u, 0x400 + i);
                   if (sb == 0 && qn > 0 && ok)                           // O_i of the previous item read out?
@@ -822,7 +846,11 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                   issue_pv(t_tile + b * kSubN, kv_lo(lv) + ((sb & 1) ? 2u * kVStep : 0u), sb > 0);
                   tc_commit(b_od);
                   if (sb == nsb - 1) tc_commit(b_ofin);
-                  if (sb + kNB < nsb) ok = qk_step(sb + kNB, b);
+                  if constexpr (C::kWide) {
+                    if ((sb & 1) && sb + 3 < nsb) ok = qk_step(sb + 3, b - 1);
+                  } else if (sb + kNB < nsb) {
+                    ok = qk_step(sb + kNB, b);
+                  }
                   if ((sb & 1) || sb == nsb - 1) kv_release(lv);
                   b = (b + 1 == kNB) ? 0 : b + 1;
                 }
