@@ -137,6 +137,8 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
   const int slice = work / a.row_blocks;
   const int row0 = (work - slice * a.row_blocks) * C::kRows;
   const int D = kExact ? W : a.head_dim, Sk = a.seqlen_k;
+  start_after_predecessor();
+  let_successor_start();
   // An earlier launch's expired wait is still in the status word: leave O alone, tell the host
   // (as the prefill kernel does).  The barriers below are passed all the same.
   const bool stale = __any_sync(0xffffffffu, a.status != nullptr && *reinterpret_cast<volatile int*>(a.status) != 0);
@@ -468,13 +470,13 @@ cudaError_t launch_decode_inst(DecodeArgs a, int sms, cudaStream_t stream) {
   cfg.blockDim = dim3(32 * warps, 1, 1);
   cfg.dynamicSmemBytes = C::smem_bytes(warps);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(a.n_split);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2] = {overlap_attribute()};
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(a.n_split);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = a.n_split > 1 ? 1 : 0;
+  cfg.numAttrs = a.n_split > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 

@@ -89,6 +89,14 @@ int current_sm_count(cudaError_t* e);
 // the warps of each in *warps.  Host arithmetic only.
 int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int* warps);
 
+// Launch attribute of every kernel that calls start_after_predecessor().
+inline cudaLaunchAttribute overlap_attribute() {
+  cudaLaunchAttribute a{};
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+
 // The work plan launch_fwd would choose on a GPU of `sms` SMs: fills rows_per_item, n_pairs,
 // fold and n_units of `a` from its seqlen, seqlen_k and n_slices.  Host arithmetic only.
 // head_dim is the kernel's (64, 128 or 256); false for any other or for sms <= 0.

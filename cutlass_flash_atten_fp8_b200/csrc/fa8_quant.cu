@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(kSegThreads, 2) segment_kernel(const uint4* __
                                                                  uint8_t* __restrict__ tail_out, int n_tail, int csize,
                                                                  float* __restrict__ amax, float* __restrict__ descale) {
   __shared__ float peers[8];
+  start_after_predecessor();
   const int seg = blockIdx.x / csize, rank = blockIdx.x - seg * csize;
   x += seg * n_vec;
   y += seg * n_vec;
@@ -238,6 +239,8 @@ template <bool kBf16>
 __global__ void __launch_bounds__(kQuantThreads, 8) amax_kernel(const uint4* __restrict__ x, int64_t n_vec,
                                                             const uint16_t* __restrict__ tail, int n_tail,
                                                             float* __restrict__ amax) {
+  start_after_predecessor();
+  let_successor_start();
   x += blockIdx.y * n_vec;
   amax += blockIdx.y;
   AbsMax<kBf16> mx;
@@ -260,6 +263,7 @@ __global__ void __launch_bounds__(kQuantThreads, 8) cast_kernel(const uint4* __r
                                                             uint8_t* __restrict__ tail_out, int n_tail,
                                                             const float* __restrict__ amax,
                                                             float* __restrict__ descale) {
+  start_after_predecessor();
   x += blockIdx.y * n_vec;
   y += blockIdx.y * n_vec;
   const float a = amax[blockIdx.y];
@@ -286,13 +290,13 @@ cudaError_t launch_segments(const uint4* x, uint2* y, int64_t n_vec, const uint1
   cfg.gridDim = dim3(static_cast<unsigned>(n_seg) * csize, 1, 1);
   cfg.blockDim = dim3(threads, 1, 1);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = csize;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2] = {overlap_attribute()};
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = csize;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = csize > 1 ? 1 : 0;
+  cfg.numAttrs = csize > 1 ? 2 : 1;
   return cudaLaunchKernelEx(&cfg, &segment_kernel<kBf16>, x, y, n_vec, tail_in, tail_out, n_tail, csize, amax, descale);
 }
 
@@ -341,9 +345,17 @@ cudaError_t launch_two_pass(const uint4* x, uint2* y, int64_t n_vec, const uint1
   const dim3 grid(static_cast<unsigned>(want < 1 ? 1 : (want > cap ? cap : want)), static_cast<unsigned>(n_seg), 1);
   cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(float) * n_seg, stream);
   if (e != cudaSuccess) return e;
-  amax_kernel<kBf16><<<grid, kQuantThreads, 0, stream>>>(x, n_vec, tail_in, n_tail, amax);
-  cast_kernel<kBf16><<<grid, kQuantThreads, 0, stream>>>(x, y, n_vec, tail_in, tail_out, n_tail, amax, descale);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kQuantThreads, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1] = {overlap_attribute()};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  e = cudaLaunchKernelEx(&cfg, &amax_kernel<kBf16>, x, n_vec, tail_in, n_tail, amax);
+  if (e != cudaSuccess) return e;
+  return cudaLaunchKernelEx(&cfg, &cast_kernel<kBf16>, x, y, n_vec, tail_in, tail_out, n_tail, static_cast<const float*>(amax),
+                            descale);
 }
 
 // Which form (us, fp16, measured on segments of the given size):

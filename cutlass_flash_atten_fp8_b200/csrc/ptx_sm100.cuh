@@ -301,6 +301,14 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
   return r;
 }
 
+// ------------------------------------------------------------ launch overlap --
+// Kernels of this library may be started before the one ahead of them in the stream has finished
+// (programmatic stream serialisation).  start_after_predecessor() returns once that one, and with
+// it everything before it, is complete and its writes are visible: nothing in global memory is
+// touched before.  let_successor_start() allows the next one's CTAs onto SMs that are free.
+__device__ __forceinline__ void start_after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ------------------------------------------------------------ scalar math --
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
