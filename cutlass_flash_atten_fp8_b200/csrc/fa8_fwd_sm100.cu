@@ -108,11 +108,11 @@ struct Cfg {
   // Query tiles per CTA: two, or one where O alone takes half of tensor memory (head_dim 256).
   static constexpr int kTiles = (D <= 128) ? 2 : 1;
   // Softmax warps per 32-row group of a tile: they take the sub-blocks in turn, warp j the
-  // sub-blocks j, j + kW, ...  Two per group; at head_dim 256 that leaves eight of the sixteen
-  // softmax warps without work (four per group on the one tile measured 25 % slower: the
-  // hand-over of P is ordered, so more warps per group only lengthen that chain).
+  // sub-blocks j, j + kW, ...  Two per group; four on the one tile of head_dim 256 (B2 H16 S4096:
+  // 255 us against 261, S1024 88.6 against 92).  Not more than score buffers: a warp tells the phases of a buffer's barriers apart by
+  // their parity.
 #ifndef FA8_D256_KW
-#define FA8_D256_KW 2
+#define FA8_D256_KW 4
 #endif
   static constexpr int kW = (D == 256) ? FA8_D256_KW : 2;
   // Score buffers per tile, 64 fp32 columns each, used round robin (sub-block sb in buffer
@@ -700,12 +700,19 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         // keys is 32 rows further down.
         constexpr uint32_t kVStep = kVNatural ? (32u * C::kBlkD / 16u) : 2u;   // descriptor units per 32 keys
         constexpr uint32_t kKHalf = kSubN * C::kBlkD / 16;                     // rows 64..127 of a K tile
+        // Column blocks of 128: k-steps of QK and output columns of the second block follow the true
+        // head_dim (160, 192, 224 run on the 256 kernel).
+        const int d_steps = (args.head_dim + 31) >> 5;
+        const uint32_t idesc_pv1 =
+            C::kNBlk > 1 ? umma_idesc(kTileM, 32 * d_steps - 128, kFmt) | (kVNatural ? (1u << 16) : 0u) : kIdescPV;
         // S_i[h] = Q_i K_sb^T: D/32 steps of K = 32 bytes along the swizzled rows.
         auto issue_qk = [&](uint32_t ts, uint32_t q_lo, uint32_t k_lo) {
   #pragma unroll
           for (int k = 0; k < D / 32; ++k) {
             // K-step k lies in column block k / 4 (four steps of 32 bytes per 128-byte row)
             const uint32_t off = (C::kNBlk > 1 ? (k >> 2) * kBlk16 : 0u) + 2u * (C::kNBlk > 1 ? (k & 3) : k);
+            // (at head_dim 256, whose tensor side is what limits) columns past the true head_dim are zeros
+            if (C::kNBlk > 1 && k > 4 && k >= d_steps) break;
             mma_f8_ss(ts, make_desc(q_lo + off, qk_hi), make_desc(k_lo + off, qk_hi), kIdescQK, k > 0);
           }
         };
@@ -715,8 +722,8 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           for (int nb = 0; nb < C::kNBlk; ++nb)         // 128 output columns per MMA: one column block of V
   #pragma unroll
             for (int k = 0; k < kSubN / 32; ++k)
-              mma_f8_ts(t_o + nb * C::kBlkD, ts + 8u * k, make_desc(v_lo + nb * kBlk16 + kVStep * k, v_hi), kIdescPV,
-                        (acc || k > 0) ? 1u : 0u);
+              mma_f8_ts(t_o + nb * C::kBlkD, ts + 8u * k, make_desc(v_lo + nb * kBlk16 + kVStep * k, v_hi),
+                        nb == 0 ? kIdescPV : idesc_pv1, (acc || k > 0) ? 1u : 0u);
         };
         auto kv_wait = [&](uint32_t load) {
           const uint32_t slot = load & kSlotMask;

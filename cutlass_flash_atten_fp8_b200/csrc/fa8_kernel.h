@@ -106,7 +106,9 @@ bool plan_fwd(int head_dim, bool causal, KernelArgs& a, int sms);
 #ifndef FA8_EPI_COLS_128
 #define FA8_EPI_COLS_128 16
 #endif
-constexpr int epi_cols(int kernel_head_dim) { return kernel_head_dim == 128 ? FA8_EPI_COLS_128 : 32; }
+constexpr int epi_cols(int kernel_head_dim) {
+  return kernel_head_dim == 128 ? FA8_EPI_COLS_128 : (kernel_head_dim == 256 ? 16 : 32);
+}
 
 // One warp waits (bounded by limit_ns) on a barrier that never completes; see fa8_selftest_expired_wait.
 cudaError_t launch_expired_wait(int* status, int* host_status, unsigned long long limit_ns, cudaStream_t stream);
