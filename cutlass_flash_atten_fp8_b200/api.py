@@ -180,7 +180,7 @@ def quantize_e4m3(x: torch.Tensor, per_head: bool = False):
     """Amax quantisation of a contiguous fp16 / bf16 CUDA tensor: returns (x8, descale) with
     x8 = e4m3(x * 448 / max|x|) shaped like x and x ~= descale * x8.  Per tensor, descale is a
     one-element fp32 tensor; with per_head=True x is [batch, heads, ...] and every (batch,
-    head) slice gets its own scale: descale is [batch*heads].  Stream-ordered, two HBM-bound
+    head) slice gets its own scale: descale is [batch*heads].  Stream-ordered, HBM-bound
     kernels; stands where the reference's callers cast with torch (test.py:20-22, 68-70)."""
     native = _native()
     if native:

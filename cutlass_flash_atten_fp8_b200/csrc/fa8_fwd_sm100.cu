@@ -9,18 +9,19 @@
 // each being two 128-row query tiles of one (batch, head) slice (one tile at head_dim
 // 256), and walks the key/value sequence; K and V^T arrive as 128-position tiles, the
 // arithmetic runs on 64-position sub-blocks so that each query tile has two (head_dim
-// 64: three) score buffers in tensor memory and its next S = Q K^T is computed while
+// 64: three, 256: four) score buffers in tensor memory and its next S = Q K^T is computed while
 // the softmax of the current sub-block is still running:
 //
 //   warp 18     TMA producer: Q tiles (double-buffered across work items), then K_j /
 //               V_j tiles into a ring of shared-memory slots, each guarded by a
 //               full/empty mbarrier pair.
 //   warps 16,17 MMA issuers, one per query tile (one elected lane each):
-//               S_i[sb % kSBuf] = Q_i K_sb^T (M128 N64) and O_i += P_i(sb) V_sb
+//               S_i[sb % kSBuf] = Q_i K_sb^T (M128 N64; head_dim 256: N128) and O_i += P_i(sb) V_sb
 //               (M128 N=head_dim) as tcgen05.mma kind::f8f6f4 with fp32 accumulators
 //               in tensor memory; completion is signalled with tcgen05.commit on
 //               mbarriers.
-//   warps 0-7   online softmax for query tile 0, warps 8-15 for tile 1.  A TMEM lane
+//   warps 0-7   online softmax for query tile 0, warps 8-15 for tile 1 (head_dim 256: all
+//               sixteen for the one tile).  A TMEM lane
 //               is a query row (tcgen05.ld 32x32b: one row per thread, no shuffles).
 //               Warps w and w+4 of a tile own the same 32 rows and take the sub-blocks
 //               in turn, so four softmax warps per scheduler keep the special-function
@@ -109,12 +110,9 @@ struct Cfg {
   static constexpr int kTiles = (D <= 128) ? 2 : 1;
   // Softmax warps per 32-row group of a tile: they take the sub-blocks in turn, warp j the
   // sub-blocks j, j + kW, ...  Two per group; four on the one tile of head_dim 256 (B2 H16 S4096:
-  // 255 us against 261, S1024 88.6 against 92).  Not more than score buffers: a warp tells the phases of a buffer's barriers apart by
-  // their parity.
-#ifndef FA8_D256_KW
-#define FA8_D256_KW 4
-#endif
-  static constexpr int kW = (D == 256) ? FA8_D256_KW : 2;
+  // 255 us against 261, S1024 88.6 against 92).  Not more than score buffers: a warp tells the
+  // phases of a buffer's barriers apart by their parity.
+  static constexpr int kW = (D == 256) ? 4 : 2;
   // Score buffers per tile, 64 fp32 columns each, used round robin (sub-block sb in buffer
   // sb % kSBuf).  A tile owns 512 / kTiles columns of tensor memory:
   //   head_dim  64: 3 x 64 + 64  = 256;  with three buffers the score of a warp's next sub-block
@@ -135,6 +133,7 @@ struct Cfg {
   // keys, 291; PV at N256, no change.)
   static constexpr bool kWide = D == 256;
   static_assert(!kWide || (kTiles == 1 && kSBuf == 4), "the order of loads and products is written for one tile and four buffers");
+  static_assert(kW <= kSBuf, "see kW");
   static_assert(kOCol + D <= kTileCols, "tensor-memory budget");
   static_assert(4 * kW * kTiles <= 16, "sixteen softmax warps");
   static constexpr int kSlots = (D == 128) ? 8 : (D == 64 ? 16 : 4);   // ring slots, one K or V tile each

@@ -148,8 +148,8 @@ int fa8_quantize_e4m3_segments(const void* src, int32_t src_dtype, void* dst, in
  * that is being captured into a graph, where cudaMalloc is an error - has no such buffer to give.
  * Here the maxima live in a file-scope device array of the library: FA8_NOALLOC_MAX_SEGMENTS
  * floats (16 KB), present on every GPU that loads the library until the process ends.  The call
- * allocates nothing, neither with cudaMalloc nor through any library: it clears the n_seg entries it
- * needs (stream-ordered) and enqueues the two passes on `cuda_stream`; src, dst and descale are the
+ * allocates nothing, neither with cudaMalloc nor through any library: it enqueues its passes on
+ * `cuda_stream`, which write the n_seg entries before they read them; src, dst and descale are the
  * caller's, as before (descale must not be NULL: it is the only way the scales come out).
  *   - n_seg above FA8_NOALLOC_MAX_SEGMENTS is refused with FA8_ERR_UNSUPPORTED (the detail
  *     string names both numbers); seg_len a multiple of 8 unless n_seg is 1.
@@ -183,7 +183,10 @@ int fa8_supported(int32_t seqlen_k, int32_t head_dim, int32_t v_layout);
  * items of 256 query rows (two 128-row tiles side by side; one tile at head dims above 128);
  * a causal unit pairs item f with item n-1-f of a slice so that all units cost the same.
  * Problems that would leave more than half of the SMs idle are cut finer: items of 128 rows,
- * or causal items as units of their own.  Results do not depend on the plan.
+ * or causal items as units of their own.  Results do not depend on the plan.  (Launches without a
+ * causal mask whose query heads share key/value heads are first regrouped, slices = batch *
+ * heads_kv of heads / heads_kv * seqlen rows, where that needs fewer 128-row tiles; those of fewer than
+ * 64 such rows with natural V may go to the decode kernel, which splits the keys instead.)
  * plan[0] = query rows per item, plan[1] = 1 if causal items are paired, plan[2] = items per
  * slice, plan[3] = units (the grid is min(units, sm_count) CTAs).  seqlen_k 0 = seqlen. */
 int fa8_work_plan(int32_t slices, int32_t seqlen, int32_t seqlen_k, int32_t head_dim, int32_t is_causal,
