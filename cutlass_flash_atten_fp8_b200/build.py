@@ -94,8 +94,12 @@ def binding_is_stale() -> bool:
     hp = out + ".srchash"
     if not os.path.exists(out) or not os.path.exists(hp):
         return True
+    try:
+        now = _binding_digest()
+    except FileNotFoundError:
+        return False          # an installed copy without its sources cannot go stale
     with open(hp) as f:
-        return f.read().strip() != _binding_digest()
+        return f.read().strip() != now
 
 
 def _binding_digest() -> str:

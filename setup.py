@@ -44,6 +44,7 @@ class BuildNative(build_ext):
         shutil.copy2(lib, dst_pkg)
         shutil.copy2(b.HASH_PATH, dst_pkg)
         shutil.copy2(module, self.build_lib)
+        shutil.copy2(module + ".srchash", self.build_lib)      # without it the package takes the module for stale
 
 
 setup(

@@ -1,0 +1,40 @@
+"""When the package's operators go through the compiled module, without a GPU."""
+import pytest
+import torch
+
+from cutlass_flash_atten_fp8_b200 import api, build
+
+F8 = torch.float8_e4m3fn
+
+
+def test_module_is_taken_when_built_and_left_alone_when_stale(monkeypatch):
+    build.build_binding()
+    assert not build.binding_is_stale()
+    monkeypatch.setattr(api, "_native_module", None)
+    assert api._native() and hasattr(api._native(), "_forward")
+    monkeypatch.setattr(build, "_binding_digest", lambda: "0" * 64)
+    assert build.binding_is_stale()
+    monkeypatch.setattr(api, "_native_module", None)
+    assert api._native() is False
+
+
+def test_an_installed_copy_without_sources_is_not_stale(monkeypatch):
+    build.build_binding()
+
+    def gone():
+        raise FileNotFoundError
+    monkeypatch.setattr(build, "_binding_digest", gone)
+    assert not build.binding_is_stale()
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_the_same_complaints_either_way(monkeypatch, native):
+    build.build_binding()
+    monkeypatch.setattr(api, "_native_module", None if native else False)
+    q = torch.zeros(1, 1, 128, 64).to(F8)
+    with pytest.raises(RuntimeError, match="q must be a CUDA tensor"):
+        api.flash_attention_v2_cutlass(q, q, q, False, 0.125, v_layout="natural")
+    with pytest.raises(RuntimeError, match="q must be a CUDA tensor"):
+        api.flash_attention_v2_cutlass(q, q, q, False, 0.125, v_layout="upside down")
+    with pytest.raises(RuntimeError, match="x must be a CUDA tensor"):
+        api.quantize_e4m3(torch.zeros(4, 4, dtype=torch.float16))
