@@ -85,9 +85,9 @@ bool decode_takes(int64_t slices, int64_t rows, int seqlen_k, int head_dim, int 
 // SMs of the current device (kept per device); 0 and *e on failure.
 int current_sm_count(cudaError_t* e);
 
-// How launch_decode splits the keys of `items` (slices times row blocks): CTAs per cluster, and
+// How launch_decode splits the keys of `items` (slices times row blocks): CTAs per cluster (at most max_split), and
 // the warps of each in *warps.  Host arithmetic only.
-int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int* warps);
+int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int max_split, int* warps);
 
 // Launch attribute of every kernel that calls start_after_predecessor().
 inline cudaLaunchAttribute overlap_attribute() {
