@@ -21,7 +21,7 @@ LIB_PATH = os.path.join(PKG_DIR, "libfa8_b200.so")
 # file contents but not necessarily modification times, so staleness is decided by content.
 HASH_PATH = os.path.join(PKG_DIR, "libfa8_b200.srchash")
 SOURCES = ["fa8_fwd_sm100.cu", "fa8_decode_sm100.cu", "fa8_quant.cu", "fa8_capi.cu"]
-HEADERS = ["fa8_kernel.h", "ptx_sm100.cuh", os.path.join(REPO_DIR, "include", "fa8_b200.h")]
+HEADERS = ["fa8_kernel.h", "phase_rule.h", "ptx_sm100.cuh", os.path.join(REPO_DIR, "include", "fa8_b200.h")]
 
 
 def nvcc_path() -> str:

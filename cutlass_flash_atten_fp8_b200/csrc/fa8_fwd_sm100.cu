@@ -58,6 +58,7 @@
 #include <cstdint>
 
 #include "fa8_kernel.h"
+#include "phase_rule.h"
 #include "ptx_sm100.cuh"
 
 namespace fa8 {
@@ -110,8 +111,7 @@ struct Cfg {
   static constexpr int kTiles = (D <= 128) ? 2 : 1;
   // Softmax warps per 32-row group of a tile: they take the sub-blocks in turn, warp j the
   // sub-blocks j, j + kW, ...  Two per group; four on the one tile of head_dim 256 (B2 H16 S4096:
-  // 255 us against 261, S1024 88.6 against 92).  Not more than score buffers: a warp tells the
-  // phases of a buffer's barriers apart by their parity.
+  // 255 us against 261, S1024 88.6 against 92).  Not more than score buffers: see phase_rule.h.
   static constexpr int kW = (D == 256) ? 4 : 2;
   // Score buffers per tile, 64 fp32 columns each, used round robin (sub-block sb in buffer
   // sb % kSBuf).  A tile owns 512 / kTiles columns of tensor memory:
@@ -133,7 +133,7 @@ struct Cfg {
   // keys, 291; PV at N256, no change.)
   static constexpr bool kWide = D == 256;
   static_assert(!kWide || (kTiles == 1 && kSBuf == 4), "the order of loads and products is written for one tile and four buffers");
-  static_assert(kW <= kSBuf, "see kW");
+  static_assert(kW <= kSBuf, "see phase_rule.h");
   static_assert(kOCol + D <= kTileCols, "tensor-memory budget");
   static_assert(4 * kW * kTiles <= 16, "sixteen softmax warps");
   static constexpr int kSlots = (D == 128) ? 8 : (D == 64 ? 16 : 4);   // ring slots, one K or V tile each
@@ -159,10 +159,10 @@ struct Cfg {
   static constexpr int kEpiOffset = kQBytes + kRingBytes;
   static constexpr int kBarOffset = kEpiOffset + kEpiWarps * kEpiBytes;
   // row-group scratch shared by the warps of a 32-row group, see RowGroupShared
-  static constexpr int kGroups = 16 / kW;          // one per 32-row group of a tile slot (slot 1 idles at head_dim 256)
+  static constexpr int kGroups = 16 / kW;          // one per 32-row group of a tile
   static constexpr int kGroupBytes = kGroups * (160 + 512 * kW);
   static constexpr int kNumBars = 4 /*q_full*/ + 4 /*q_empty*/ + 2 * kSlots + 8 /*s_full*/ + 8 /*p_full*/ +
-                                  2 /*o_done*/ + 2 /*o_final*/ + 2 /*o_free*/ + 2 /*drain*/;
+                                  8 /*o_done*/ + 2 /*o_final*/ + 2 /*o_free*/ + 2 /*drain*/;
   static constexpr int kSmemBytes = kBarOffset + kNumBars * 8 + 16 /*tmem ptr, abort*/ + kGroupBytes + 1024 /*align*/;
   // Q and K rows are D bytes long: one 128-byte swizzle row for D=128, a 64-byte one for D=64.
   static constexpr uint32_t kQKLayout = (D >= 128) ? 2u : 4u;   // UMMA SWIZZLE_128B / SWIZZLE_64B
@@ -493,7 +493,8 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   const uint32_t b_q_full = take(4), b_q_empty = take(4);            // [tile][stage]
   const uint32_t b_kv_full = take(C::kSlots), b_kv_empty = take(C::kSlots);
   const uint32_t b_s_full = take(8), b_p_full = take(8);             // [tile][S buffer]
-  const uint32_t b_o_done = take(2), b_o_final = take(2), b_o_free = take(2);
+  const uint32_t b_o_done = take(8);                                  // [tile][S buffer]
+  const uint32_t b_o_final = take(2), b_o_free = take(2);
   const uint32_t bar_drain = take(2);
   auto bar_q_full = [&](int i, int st) { return b_q_full + 8u * (2 * i + st); };
   auto bar_q_empty = [&](int i, int st) { return b_q_empty + 8u * (2 * i + st); };
@@ -502,11 +503,13 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
   auto bar_s_full = [&](int i, int b) { return b_s_full + 8u * (C::kSBuf * i + b); };
   // One P barrier per S buffer: the four warps (one per 32-row group) that took the sub-block arrive.
   auto bar_p_full = [&](int i, int b) { return b_p_full + 8u * (C::kSBuf * i + b); };
-  // o_done[i]: one phase per PV of tile i.  o_final[i]: one phase per work item, after the
+  // o_done[i][b]: one phase per PV of tile i that takes its P from buffer b, so its phases are
+  // numbered like those of s_full and p_full (phase_rule.h says why one barrier for all PVs of the
+  // tile would not do).  o_final[i]: one phase per work item, after the
   // tile's last PV (the epilogue cannot use o_done: warps get there at different distances
   // from the end, which a parity wait cannot tell apart).  o_free[i]: one phase per work
-  // item, when all eight warps of the tile have read O out of tensor memory.
-  auto bar_o_done = [&](int i) { return b_o_done + 8u * i; };
+  // item, when all softmax warps of the tile have read O out of tensor memory.
+  auto bar_o_done = [&](int i, int b) { return b_o_done + 8u * (C::kSBuf * i + b); };
   auto bar_o_final = [&](int i) { return b_o_final + 8u * i; };
   auto bar_o_free = [&](int i) { return b_o_free + 8u * i; };
   volatile uint32_t* tmem_ptr_slot =
@@ -534,13 +537,13 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
     for (int x = 0; x < 8; ++x) {
       mbar_init(b_s_full + 8u * x, 1);
       mbar_init(b_p_full + 8u * x, 4);     // one arrive per 32-row group
+      mbar_init(b_o_done + 8u * x, 1);
     }
     for (int s = 0; s < C::kSlots; ++s) {
       mbar_init(bar_kv_full(s), 1);
       mbar_init(bar_kv_empty(s), 2);       // both MMA issuers hand a slot back
     }
     for (int i = 0; i < 2; ++i) {
-      mbar_init(bar_o_done(i), 1);
       mbar_init(bar_o_final(i), 1);
       mbar_init(bar_o_free(i), 4 * C::kW);   // one arrive per softmax warp of the tile
     }
@@ -692,7 +695,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
         const uint32_t t_o = t_tile + C::kOCol;
         const uint32_t b_sf0 = bar_s_full(i, 0), b_sf1 = bar_s_full(i, 1);
         const uint32_t b_pf0 = bar_p_full(i, 0), b_pf1 = bar_p_full(i, 1);
-        const uint32_t b_od = bar_o_done(i), b_ofin = bar_o_final(i), b_ofree = bar_o_free(i);
+        const uint32_t b_od0 = bar_o_done(i, 0), b_od1 = bar_o_done(i, 1), b_ofin = bar_o_final(i), b_ofree = bar_o_free(i);
         // The V^T tile is D rows of 128 key positions (K-major, 128-byte swizzle), of which
         // sub-block h covers bytes 64h..64h+63 of every row = K-steps 2h and 2h+1.  In the
         // natural layout the tile is 128 key rows of D bytes (swizzled like K): a K-step of 32
@@ -783,7 +786,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 pp0 ^= 1u;
                 tc_fence_after();
                 issue_pv(t_s0, v_lo, j > 0);
-                tc_commit(b_od);
+                tc_commit(b_od0);
                 if (!pv1) tc_commit(b_ofin);
                 if (qk0) {
                   issue_qk(t_s0, q_lo, k_lo);
@@ -796,7 +799,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                   pp1 ^= 1u;
                   tc_fence_after();
                   issue_pv(t_s1, v_lo + 2u * kVStep, true);
-                  tc_commit(b_od);
+                  tc_commit(b_od1);
                   if (sb + 1 == nsb - 1) tc_commit(b_ofin);
                   if (qk1) {
                     issue_qk(t_s1, q_lo, k_lo + kKHalf);
@@ -853,7 +856,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                   pp ^= 1u << b;
                   tc_fence_after();
                   issue_pv(t_tile + b * kSubN, kv_lo(lv) + ((sb & 1) ? 2u * kVStep : 0u), sb > 0);
-                  tc_commit(b_od);
+                  tc_commit(bar_o_done(i, b));
                   if (sb == nsb - 1) tc_commit(b_ofin);
                   if constexpr (C::kWide) {
                     if ((sb & 1) && sb + 3 < nsb) ok = qk_step(sb + 3, b - 1);
@@ -919,10 +922,9 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       const uint32_t s_stage = smem_base + C::kEpiOffset + static_cast<uint32_t>(warp % C::kEpiWarps) * C::kEpiBytes;
       if (lane == 0) prefetch_tensormap(&tm_o);
       // Running phases of the barriers this warp waits on.  Sub-block sb of an item uses phase
-      // number (uses of its buffer in earlier items) + sb / kNB of s_full and p_full alike; bit b
-      // of ph_bits is the parity of the first of these for buffer b.
+      // number (uses of its buffer in earlier items) + sb / kNB of s_full, p_full and o_done alike;
+      // bit b of ph_bits is the parity of the first of these for buffer b.
       uint32_t ph_bits = 0;
-      uint32_t pv_cnt = 0;         // PVs of this tile before the current item: o_done[i] base
       uint32_t items = 0;          // work items of this tile so far: o_final[i] phase, l_part buffer
       uint32_t version = 0;        // last value of grp.version this warp has seen
       bool ok = true;
@@ -965,8 +967,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           for (int sb = h; sb < tile_nsb; sb += kW) {
             const int b = sb % kNB;                          // the score buffer of this sub-block
             const uint32_t t_sb = t_tile + b * kSubN;
-            bool ok_s = wait_bounded(wctx, bar_s_full(i, b), ((ph_bits >> b) ^ static_cast<uint32_t>(sb / kNB)) & 1u,
-                                     0x500 + i);
+            bool ok_s = wait_bounded(wctx, bar_s_full(i, b), phase_parity<kNB>(ph_bits, sb), 0x500 + i);
             tc_fence_after();
             const int lim = col_lim - sb * kSubN;            // sub-block-local first masked column
 
@@ -985,9 +986,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             // P(sb) may be handed over only after P(sb-1) has been (by the warp before this one in
             // the rotation): from then on nobody else can raise the maximum before PV(sb) is issued.
             if (sb > 0) {
-              const int bp = (sb - 1) % kNB;
-              ok_s = wait_bounded(wctx, bar_p_full(i, bp),
-                                  ((ph_bits >> bp) ^ static_cast<uint32_t>((sb - 1) / kNB)) & 1u, 0x800 + i) && ok_s;
+              ok_s = wait_bounded(wctx, bar_p_full(i, (sb - 1) % kNB), phase_parity<kNB>(ph_bits, sb - 1), 0x800 + i) && ok_s;
             }
             // One vote settles the common case: waits fine, maximum unchanged, no overflow.
             // Some P above kLazyLimit implies a sum above it (all P >= 0); a false alarm only
@@ -1018,7 +1017,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
                 const float m_new = fmaxf(m, row_max(t_sb, lim));
                 if (sb > 0) {
                   // O_i must be quiescent: PV_i(sb-1) complete; PV_i(sb) waits for this warp.
-                  ok = wait_bounded(wctx, bar_o_done(i), (pv_cnt + static_cast<uint32_t>(sb - 1)) & 1u, 0x700 + i);
+                  ok = wait_bounded(wctx, bar_o_done(i, (sb - 1) % kNB), phase_parity<kNB>(ph_bits, sb - 1), 0x700 + i);
                   ok = __all_sync(0xffffffffu, ok);
                   if (!ok) break;
                   tc_fence_after();
@@ -1053,9 +1052,7 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
           }
           if (!ok) break;
   #pragma unroll
-          for (int b = 0; b < kNB; ++b)                      // buffer b served (tile_nsb - b) / kNB, rounded up, sub-blocks
-            if (((tile_nsb + kNB - 1 - b) / kNB) & 1) ph_bits ^= 1u << b;
-          pv_cnt += static_cast<uint32_t>(tile_nsb);
+          for (int b = 0; b < kNB; ++b) ph_bits ^= phases_used<kNB>(b, tile_nsb) << b;
 
           // Epilogue: O_i / l -> fp16 -> global; each warp of the group writes its share of the head dim.
           ok = wait_bounded(wctx, bar_o_final(i), items & 1u, 0x600 + i);
