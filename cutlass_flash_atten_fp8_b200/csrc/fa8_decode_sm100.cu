@@ -153,8 +153,9 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
   const int step_lo = static_cast<int>(static_cast<int64_t>(n_steps) * rank / n_split);
   const int step_hi = static_cast<int>(static_cast<int64_t>(n_steps) * (rank + 1) / n_split);
 
-  // Rows past the last key are read as the last key again (its memory is there, its score is
-  // masked): no branch around a load.  Columns past head_dim are zeros.
+  // Rows past the last key are read as the last key again (its memory is there): no branch around a
+  // load.  The scores of such keys are masked and their values cleared before use, for the last
+  // key's may be an infinity.  Columns past head_dim are zeros.
   const int k_col = 16 * t, v_col = (C::kVWords * 4) * g;
   auto load_k = [&](uint4 (&r)[C::kChunks], int key) {
     const uint8_t* p = kp + static_cast<size_t>(min(key, Sk - 1)) * D + k_col;
@@ -164,11 +165,12 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
       if (kExact || 64 * c + k_col < D) r[c] = ld_stream16(p + 64 * c);
     }
   };
+  auto v_key = [&](int key0, int i) { return key0 + 16 * (i >> 2) + 8 * ((i >> 1) & 1) + 2 * t + (i & 1); };
   auto load_v = [&](uint32_t (&r)[8][C::kVWords], int key0, int blk) {
     const int col = 128 * blk + v_col;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {                       // k word i / 4, byte i % 4
-      const int key = key0 + 16 * (i >> 2) + 8 * ((i >> 1) & 1) + 2 * t + (i & 1);
+      const int key = v_key(key0, i);
       const uint8_t* p = vp + static_cast<size_t>(min(key, Sk - 1)) * D + col;
 #pragma unroll
       for (int w = 0; w < C::kVWords; ++w) r[i][w] = 0u;
@@ -348,6 +350,13 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
       }
 #pragma unroll
       for (int blk = 0; blk < C::kVBlocks; ++blk) {
+        if (key0 + kStepKeys > Sk) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int w = 0; w < C::kVWords; ++w)
+              if (v_key(key0, i) >= Sk) vr[i][w] = 0u;
+        }
 #pragma unroll
         for (int w = 0; w < C::kVWords; ++w) {
 #pragma unroll

@@ -93,3 +93,16 @@ def test_a_stale_status_word_leaves_the_output_alone():
     flash_attention_v2_cutlass(q, k, v, False, 0.125, v_layout="natural", out=out, _status=word)
     check_status(d, word=word)
     assert not bool((out == 7.0).any())
+
+
+@pytest.mark.parametrize("D,col", [(32, 5), (64, 63), (96, 40), (128, 0), (192, 150), (256, 255)])
+@pytest.mark.parametrize("Sk", [1, 33, 70, 999])
+def test_an_infinite_value_of_the_last_key_comes_through(D, col, Sk):
+    # keys past the last one take no part: 0 * inf there would be a NaN
+    q, k, v = (rand8(1, 1, s, D, seed=s, dtype=torch.float8_e5m2) for s in (1, Sk, Sk))
+    plain, _ = call(q, k, v, 0.01)
+    v[0, 0, Sk - 1, col] = float("inf")
+    out, _ = call(q, k, v, 0.01)
+    assert float(out[0, 0, 0, col]) == math.inf
+    plain[0, 0, 0, col] = math.inf
+    assert torch.equal(out, plain)
