@@ -85,18 +85,6 @@ __device__ __forceinline__ uint32_t round2(float a, float b) {
   return r;
 }
 
-// Keys and values are read once: no reason to keep them in the first-level cache.
-__device__ __forceinline__ uint4 ld_stream16(const uint8_t* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-  return v;
-}
-__device__ __forceinline__ uint2 ld_stream8(const uint8_t* p) {
-  uint2 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-  return v;
-}
-
 // Head dims up to W run in the instance built for W; bytes past head_dim are zeros in registers.
 // RB: blocks of eight query rows a CTA works on (16 rows need a second PV product per column
 // block; at W = 256 their accumulators do not fit the registers).
@@ -195,7 +183,7 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
 #pragma unroll
     for (int c = 0; c < C::kChunks; ++c) {
       uint4 x = make_uint4(0u, 0u, 0u, 0u);
-      if (row < a.rows && 64 * c + k_col < D) x = __ldg(reinterpret_cast<const uint4*>(p + 64 * c));
+      if (row < a.rows && 64 * c + k_col < D) x = ld_global(reinterpret_cast<const uint4*>(p + 64 * c));
       widen4<kE5M2>(x.x, qa[4 * c][h][0], qa[4 * c][h][1]);
       widen4<kE5M2>(x.y, qa[4 * c + 1][h][0], qa[4 * c + 1][h][1]);
       widen4<kE5M2>(x.z, qa[4 * c + 2][h][0], qa[4 * c + 2][h][1]);
@@ -236,11 +224,11 @@ __global__ void __launch_bounds__(32 * DCfg<W, RB>::kMaxWarps, 1) fa8_decode_ker
   auto row_scale = [&](int row) {
     float x = 1.f;
     if (a.descale_q != nullptr)
-      x *= __ldg(a.descale_q + (a.descale_per_head ? static_cast<size_t>(slice) * a.group + min(row, a.rows - 1) / a.seqlen_q : 0));
-    if (a.descale_k != nullptr) x *= __ldg(a.descale_k + (a.descale_per_head ? slice : 0));
+      x *= ld_global(a.descale_q + (a.descale_per_head ? static_cast<size_t>(slice) * a.group + min(row, a.rows - 1) / a.seqlen_q : 0));
+    if (a.descale_k != nullptr) x *= ld_global(a.descale_k + (a.descale_per_head ? slice : 0));
     return x;
   };
-  if (a.descale_v != nullptr) o_mul *= __ldg(a.descale_v + (a.descale_per_head ? slice : 0));
+  if (a.descale_v != nullptr) o_mul *= ld_global(a.descale_v + (a.descale_per_head ? slice : 0));
 #pragma unroll
   for (int h = 0; h < RB; ++h) {
     c_row[h] = a.scale_log2 * row_scale(row0 + g + 8 * h);

@@ -911,9 +911,9 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
       // (batch, key/value head) for K and V, re-read for every work item.
       float qk_descale = 1.f, o_scale = args.o_scale;
       if (!args.descale_per_head) {
-        if (args.descale_q != nullptr) qk_descale *= __ldg(args.descale_q);
-        if (args.descale_k != nullptr) qk_descale *= __ldg(args.descale_k);
-        if (args.descale_v != nullptr) o_scale *= __ldg(args.descale_v);
+        if (args.descale_q != nullptr) qk_descale *= ld_global(args.descale_q);
+        if (args.descale_k != nullptr) qk_descale *= ld_global(args.descale_k);
+        if (args.descale_v != nullptr) o_scale *= ld_global(args.descale_v);
       }
       float c = args.scale_log2 * qk_descale;
       float sm_scale = args.softmax_scale * qk_descale;
@@ -948,10 +948,10 @@ fa8_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__
             o_scale = args.o_scale;
             // (rows past the last one take the last one's scale: their results are dropped)
             if (args.descale_q != nullptr)
-              qk_descale *= __ldg(args.descale_q + (args.q_fold == 1 ? w.bh : w.bh * args.q_fold + min(q_row, seqlen - 1) /
+              qk_descale *= ld_global(args.descale_q + (args.q_fold == 1 ? w.bh : w.bh * args.q_fold + min(q_row, seqlen - 1) /
                                                                                   (seqlen / args.q_fold)));
-            if (args.descale_k != nullptr) qk_descale *= __ldg(args.descale_k + kv_bh);
-            if (args.descale_v != nullptr) o_scale *= __ldg(args.descale_v + kv_bh);
+            if (args.descale_k != nullptr) qk_descale *= ld_global(args.descale_k + kv_bh);
+            if (args.descale_v != nullptr) o_scale *= ld_global(args.descale_v + kv_bh);
             c = args.scale_log2 * qk_descale;
             sm_scale = args.softmax_scale * qk_descale;
             ek.set_scale(c);

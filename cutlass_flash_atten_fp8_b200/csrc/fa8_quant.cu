@@ -104,9 +104,11 @@ __device__ __forceinline__ float scale_of(float amax) { return amax > 0.f ? 448.
 __device__ __forceinline__ float descale_of(float amax) { return amax > 0.f ? amax / 448.f : 1.f; }
 
 // n_vec = 16-byte vectors of a segment; the n_tail elements behind them exist for a lone segment only.
+// x and tail_in are not declared __restrict__: the launch ahead may still be writing them when this one
+// starts, and const __restrict__ lets the compiler read them by the non-coherent path, ahead of the wait.
 template <bool kBf16>
-__global__ void __launch_bounds__(kSegThreads, 2) segment_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
-                                                                 int64_t n_vec, const uint16_t* __restrict__ tail_in,
+__global__ void __launch_bounds__(kSegThreads, 2) segment_kernel(const uint4* x, uint2* __restrict__ y,
+                                                                 int64_t n_vec, const uint16_t* tail_in,
                                                                  uint8_t* __restrict__ tail_out, int n_tail, int csize,
                                                                  float* __restrict__ amax, float* __restrict__ descale) {
   __shared__ float peers[8];
@@ -133,8 +135,9 @@ __global__ void __launch_bounds__(kSegThreads, 2) segment_kernel(const uint4* __
   float tail = 0.f;
   const bool has_tail = rank == 0 && threadIdx.x < n_tail;
   if (has_tail) {
-    tail = unpack_pair<kBf16>(tail_in[threadIdx.x]).x;
-    mx.pair(0, tail_in[threadIdx.x]);
+    const uint32_t w = tail_in[threadIdx.x];
+    tail = unpack_pair<kBf16>(w).x;
+    mx.pair(0, w);
   }
   float a = cta_max(mx.value());
   if (csize > 1) {
@@ -250,8 +253,8 @@ __global__ void __launch_bounds__(kQuantThreads, 8) amax_kernel(const uint4* __r
 #pragma unroll 4
   for (; i < keep_from; i += stride) mx.take(__ldcs(x + i));
 #pragma unroll 4
-  for (; i < n_vec; i += stride) mx.take(x[i]);
-  if (blockIdx.x == 0 && threadIdx.x < n_tail) mx.pair(0, tail[threadIdx.x]);
+  for (; i < n_vec; i += stride) mx.take(ld_global(x + i));
+  if (blockIdx.x == 0 && threadIdx.x < n_tail) mx.pair(0, ld_global(tail + threadIdx.x));
   const float m = cta_max(mx.value());
   // non-negative floats order like their bit patterns
   if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m));
@@ -261,12 +264,11 @@ template <bool kBf16>
 __global__ void __launch_bounds__(kQuantThreads, 8) cast_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
                                                             int64_t n_vec, const uint16_t* __restrict__ tail_in,
                                                             uint8_t* __restrict__ tail_out, int n_tail,
-                                                            const float* __restrict__ amax,
-                                                            float* __restrict__ descale) {
+                                                            const float* amax, float* __restrict__ descale) {
   start_after_predecessor();
   x += blockIdx.y * n_vec;
   y += blockIdx.y * n_vec;
-  const float a = amax[blockIdx.y];
+  const float a = ld_global(amax + blockIdx.y);           // written by amax_kernel, whose tail this kernel starts under
   const float scale = scale_of(a);
   if (blockIdx.x == 0 && threadIdx.x == 0 && descale != nullptr) descale[blockIdx.y] = descale_of(a);
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;

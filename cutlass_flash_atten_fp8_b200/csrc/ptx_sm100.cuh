@@ -309,6 +309,36 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
 __device__ __forceinline__ void start_after_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void let_successor_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Loads of what the launch ahead may have written.  A kernel that starts early is there while it is being
+// written, so the non-coherent path (ld.global.nc: __ldg, const __restrict__), which is for memory that nobody
+// writes while the kernel runs, is not for it; volatile keeps these behind start_after_predecessor().
+__device__ __forceinline__ float ld_global(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint16_t ld_global(const uint16_t* p) {
+  uint16_t v;
+  asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_global(const uint4* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+// The same past the first-level cache: data that is read once.
+__device__ __forceinline__ uint4 ld_stream16(const uint8_t* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_stream8(const uint8_t* p) {
+  uint2 v;
+  asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+
 // ------------------------------------------------------------ scalar math --
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
