@@ -13,12 +13,13 @@
 //                    distributed shared memory, what a thread read first stays in its registers
 //                    and the rest is read again while it is still in L2, so HBM sees 3 bytes per
 //                    element.
-//   whole_kernel     one long segment, one cooperative launch of the whole GPU with a grid barrier
-//                    between the passes: the first 48 MB (registers and shared memory of 148 SMs)
-//                    are read once, the rest again, last to first.
-//   amax_kernel +    several long segments, or a very long one: two passes over the tensor (5 bytes per element), the
-//   cast_kernel      second last to first.  amax is cleared before by a memset and accumulated
-//                    with atomicMax.
+//   amax_kernel +    longer segments: two passes over the tensor (5 bytes per element), the second last
+//   cast_kernel      to first.  amax is cleared before by a memset and accumulated with atomicMax.
+//
+// A long lone tensor in one launch with a barrier over the whole grid is faster (8 MB 6.6 us, 32 MB 11.5, 128 MB 50) but
+// starts only once all its CTAs fit the GPU at the same time: beside a kernel on another stream that keeps a
+// single SM busy it waits for that kernel's end (64 MB beside one block of 20 ms: 18 ms), for ever if that
+// kernel waits for this stream.  The two passes need no more than one free SM.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -40,13 +41,9 @@ namespace cg = cooperative_groups;
 // before them are read as streamed data, first to be replaced.  96 MB of a 256 MB tensor: 107.2 us; 64 MB
 // 108.3, none 112.8 (the second pass forwards, neither marked as streamed: 116.4).
 constexpr int64_t kKeep = 96ll << 16;
-// Longest lone segment of whole_kernel: 128 MB 50.5 us against 55.6 in two passes, 256 MB 111 against 107.
-constexpr int64_t kWholeMaxVec = 192ll << 16;
 constexpr int kQuantThreads = 256;     // of the two-pass kernels
 constexpr int kSegThreads = 512;       // most threads of a segment_kernel CTA
 constexpr int kHold = 8;               // 16-byte vectors of a thread that stay in registers between the passes
-constexpr int kStage = 12;             // whole_kernel: further ones that stay in shared memory
-constexpr int kStageBytes = kStage * kSegThreads * 16;
 
 template <bool kBf16>
 __device__ __forceinline__ float2 unpack_pair(uint32_t w) {
@@ -168,77 +165,6 @@ __global__ void __launch_bounds__(kSegThreads, 2) segment_kernel(const uint4* x,
 }
 
 template <bool kBf16>
-__global__ void __launch_bounds__(kSegThreads, 2) whole_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
-                                                               int64_t n_vec, const uint16_t* __restrict__ tail_in,
-                                                               uint8_t* __restrict__ tail_out, int n_tail,
-                                                               float* amax, float* __restrict__ descale) {
-  extern __shared__ uint4 stage[];                         // [kStage][thread]: every thread reads its own
-  cg::grid_group grid = cg::this_grid();
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (blockIdx.x == 0 && threadIdx.x == 0) *amax = 0.f;
-  uint4 hold[kHold];
-  AbsMax<kBf16> mx;
-#pragma unroll
-  for (int u = 0; u < kHold; ++u) {
-    const int64_t i = i0 + u * stride;
-    hold[u] = i < n_vec ? x[i] : make_uint4(0u, 0u, 0u, 0u);
-  }
-  grid.sync();                                             // amax is cleared; the loads are on their way
-#pragma unroll
-  for (int u = 0; u < kHold; ++u) mx.take(hold[u]);
-  const int64_t staged = i0 + kHold * stride, first = staged + kStage * stride;
-  if (staged < n_vec) {
-#pragma unroll
-    for (int u = 0; u < kStage; ++u) {
-      const int64_t i = staged + u * stride;
-      if (i < n_vec) {
-        const uint4 v = x[i];
-        stage[u * kSegThreads + threadIdx.x] = v;
-        mx.take(v);
-      }
-    }
-  }
-  const int64_t keep_from = n_vec - kKeep;
-  int64_t j = first;
-#pragma unroll 4
-  for (; j < keep_from; j += stride) mx.take(__ldcs(x + j));
-#pragma unroll 4
-  for (; j < n_vec; j += stride) mx.take(x[j]);
-  float tail = 0.f;
-  const bool has_tail = blockIdx.x == 0 && threadIdx.x < n_tail;
-  if (has_tail) {
-    tail = unpack_pair<kBf16>(tail_in[threadIdx.x]).x;
-    mx.pair(0, tail_in[threadIdx.x]);
-  }
-  const float m = cta_max(mx.value());
-  // non-negative floats order like their bit patterns
-  if (threadIdx.x == 0) atomicMax(reinterpret_cast<unsigned int*>(amax), __float_as_uint(m));
-  grid.sync();
-  const float a = *reinterpret_cast<volatile float*>(amax);
-  if (blockIdx.x == 0 && threadIdx.x == 0 && descale != nullptr) *descale = descale_of(a);
-  const float scale = scale_of(a);
-  if (first < n_vec) {
-#pragma unroll 4
-    for (int64_t i = first + (n_vec - 1 - first) / stride * stride; i >= first; i -= stride)
-      __stcs(y + i, cast8<kBf16>(__ldcs(x + i), scale));
-  }
-  if (staged < n_vec) {
-#pragma unroll
-    for (int u = kStage - 1; u >= 0; --u) {
-      const int64_t i = staged + u * stride;
-      if (i < n_vec) y[i] = cast8<kBf16>(stage[u * kSegThreads + threadIdx.x], scale);
-    }
-  }
-#pragma unroll
-  for (int u = 0; u < kHold; ++u) {
-    const int64_t i = i0 + u * stride;
-    if (i < n_vec) y[i] = cast8<kBf16>(hold[u], scale);
-  }
-  if (has_tail) tail_out[threadIdx.x] = static_cast<uint8_t>(cvt_e4m3x2(tail * scale, 0.f) & 0xffu);
-}
-
-template <bool kBf16>
 __global__ void __launch_bounds__(kQuantThreads, 8) amax_kernel(const uint4* __restrict__ x, int64_t n_vec,
                                                             const uint16_t* __restrict__ tail, int n_tail,
                                                             float* __restrict__ amax) {
@@ -302,43 +228,6 @@ cudaError_t launch_segments(const uint4* x, uint2* y, int64_t n_vec, const uint1
   return cudaLaunchKernelEx(&cfg, &segment_kernel<kBf16>, x, y, n_vec, tail_in, tail_out, n_tail, csize, amax, descale);
 }
 
-// CTAs of whole_kernel that the device holds at once (0 = cannot be launched), kept per device.
-template <bool kBf16>
-int whole_capacity(int dev, int sms) {
-  static std::atomic<int> known[64];                       // 1 + the capacity
-  const bool cached = dev >= 0 && dev < 64;
-  int c = cached ? known[dev].load(std::memory_order_acquire) : 0;
-  if (c == 0) {
-    int coop = 0, per_sm = 0;
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop ||
-        cudaFuncSetAttribute(&whole_kernel<kBf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, &whole_kernel<kBf16>, kSegThreads, kStageBytes) != cudaSuccess) {
-      cudaGetLastError();
-      per_sm = 0;
-    }
-    c = 1 + per_sm * sms;
-    if (cached) known[dev].store(c, std::memory_order_release);
-  }
-  return c - 1;
-}
-
-template <bool kBf16>
-cudaError_t launch_whole(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
-                         float* amax, float* descale, int capacity, cudaStream_t stream) {
-  const int64_t want = (n_vec + kSegThreads * kHold - 1) / (kSegThreads * kHold);
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(want < capacity ? want : capacity), 1, 1);
-  cfg.blockDim = dim3(kSegThreads, 1, 1);
-  cfg.dynamicSmemBytes = want <= capacity ? 0 : kStageBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, &whole_kernel<kBf16>, x, y, n_vec, tail_in, tail_out, n_tail, amax, descale);
-}
-
 template <bool kBf16>
 cudaError_t launch_two_pass(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
                             int n_seg, float* amax, float* descale, int sms, cudaStream_t stream) {
@@ -364,27 +253,15 @@ cudaError_t launch_two_pass(const uint4* x, uint2* y, int64_t n_vec, const uint1
 //   up to 512 KB a cluster holds a segment in registers: 16 x 128 KB 8.3 two-pass, 4.3 by cluster;
 //   up to 1.5 MB the second half is read again from L2, worth it when there are enough clusters to
 //   fill the GPU: 128 x 1 MB 64 -> 55, 32 x 1 MB 20.2 -> 15.7, 16 x 1 MB 14.5 -> 12.5, but 4 x 2 MB 12.4 -> 17;
-//   one long segment: 2 MB 8.4 -> 6.0, 8 MB 11.9 -> 7.2, 32 MB 19.6 -> 16.5, 128 MB 64 -> 50.5;
-//   anything longer: two passes.
+//   anything else: two passes.
 template <bool kBf16>
 cudaError_t launch_any(const uint4* x, uint2* y, int64_t n_vec, const uint16_t* tail_in, uint8_t* tail_out, int n_tail,
                        int n_seg, float* amax, float* descale, cudaStream_t stream) {
   if (n_vec <= 32 * 1024 || (n_vec <= 96 * 1024 && n_seg >= 12))
     return launch_segments<kBf16>(x, y, n_vec, tail_in, tail_out, n_tail, n_seg, amax, descale, stream);
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   const int sms = current_sm_count(&e);
   if (sms <= 0) return e;
-  if (n_seg == 1 && n_vec <= kWholeMaxVec) {
-    const int capacity = whole_capacity<kBf16>(dev, sms);
-    if (capacity > 0) {
-      e = launch_whole<kBf16>(x, y, n_vec, tail_in, tail_out, n_tail, amax, descale, capacity, stream);
-      // fewer SMs than the device has may be open to this process: then two passes
-      if (e != cudaErrorCooperativeLaunchTooLarge) return e;
-      cudaGetLastError();
-    }
-  }
   return launch_two_pass<kBf16>(x, y, n_vec, tail_in, tail_out, n_tail, n_seg, amax, descale, sms, stream);
 }
 

@@ -1,5 +1,7 @@
-"""The three forms of the quantisation (a cluster per segment, one cooperative launch, two passes) at the
-sizes where one takes over from another or a piece is not full: same bytes and scales as plain torch."""
+"""The two forms of the quantisation (a cluster per segment, two passes) at the sizes where one takes over
+from another or a piece is not full: same bytes and scales as plain torch."""
+import time
+
 import pytest
 import torch
 
@@ -18,9 +20,8 @@ def check(x, per_head):
 
 
 # elements of a lone tensor: one vector less and more than a thread's registers hold (128 x 8 and 512 x 8
-# vectors of 8), one more than a cluster's (8 x 512 x 8), what one CTA more needs, one vector more than
-# all CTAs' registers hold (296 x 512 x 8), than registers and shared memory (296 x 512 x 20), and past the
-# longest one-launch tensor
+# vectors of 8), one more than a cluster's (8 x 512 x 8), and sizes of one vector more than a power of two or a full grid
+# up to more than stays in L2
 @pytest.mark.parametrize("n", [1, 7, 9, 8191, 8200, 32768 + 8, 262144, 262144 + 13, 9699328 + 9, 24248320 + 8, 24248320 * 2 + 3,
                                192 * 2 ** 19 + 11])
 def test_lone_tensors(n):
@@ -49,3 +50,23 @@ def test_lone_zeros_and_nan():
         x[n // 3], x[n // 2] = float("nan"), 2.0
         y, descale = quantize_e4m3(x)
         assert bool(y.float()[n // 3].isnan()) and float(y.float()[n // 2]) == 448.0 and abs(float(descale) * 224.0 - 1.0) < 1e-6
+
+
+@pytest.mark.parametrize("shape,per_head", [((1, 1, 1000, 64), False), ((1, 16, 2048, 128), False), ((1, 32, 8192, 128), False),
+                                            ((4, 32, 2048, 128), True), ((4, 32, 4096, 128), True), ((1, 4, 8192, 128), True)])
+def test_a_long_kernel_elsewhere_is_not_waited_for(shape, per_head):
+    # one block that keeps a little of one SM for about 0.2 s on another stream; in a serving process it could be
+    # waiting for this stream
+    x = torch.randn(shape, device="cuda").to(torch.float16)
+    quantize_e4m3(x, per_head=per_head)
+    torch.cuda.synchronize()
+    side, asleep, done = torch.cuda.Stream(), torch.cuda.Event(), torch.cuda.Event()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(400_000_000)
+        asleep.record()
+    time.sleep(0.01)
+    quantize_e4m3(x, per_head=per_head)
+    done.record()
+    done.synchronize()
+    assert not asleep.query()
+    torch.cuda.synchronize()
