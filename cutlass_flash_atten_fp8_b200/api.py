@@ -11,6 +11,7 @@ from __future__ import annotations
 
 import ctypes
 import importlib.util
+import warnings
 from typing import List, Optional
 
 import torch
@@ -23,16 +24,21 @@ _native_module = None        # the compiled module once asked for, False where i
 
 def _native():
     """The compiled torch module (csrc/torch_binding.cpp), whose _forward and _quantize take the calls
-    that nothing is wrong with.  False where it is missing or older than its source: every call is
-    then made from here, through ctypes."""
+    that nothing is wrong with.  False where it is missing, older than its source, built for another
+    torch or not to be loaded: every call is then made from here, through ctypes, which depends on
+    the library only."""
     global _native_module
     if _native_module is None:
         _lib.load()              # raises if the library itself is missing or stale
         module = False
         if not build.binding_is_stale():
-            spec = importlib.util.spec_from_file_location(build.BINDING_NAME, build.binding_path())
-            module = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(module)
+            try:
+                spec = importlib.util.spec_from_file_location(build.BINDING_NAME, build.binding_path())
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+            except (ImportError, OSError) as e:
+                warnings.warn(f"{build.binding_path()} cannot be loaded ({e}); calls go through ctypes")
+                module = False
         _native_module = module
     return _native_module
 

@@ -90,16 +90,21 @@ def binding_path() -> str:
 
 
 def binding_is_stale() -> bool:
+    """True when the module is missing, was built from other sources than the ones present, or against
+    another torch than the one installed: it links torch's own libraries."""
+    import torch
     out = binding_path()
     hp = out + ".srchash"
     if not os.path.exists(out) or not os.path.exists(hp):
         return True
-    try:
-        now = _binding_digest()
-    except FileNotFoundError:
-        return False          # an installed copy without its sources cannot go stale
     with open(hp) as f:
-        return f.read().strip() != now
+        built = f.read().split()
+    if len(built) != 2 or built[1] != str(torch.__version__):
+        return True
+    try:
+        return built[0] != _binding_digest()
+    except FileNotFoundError:
+        return False          # an installed copy without its sources cannot go stale by them
 
 
 def _binding_digest() -> str:
@@ -147,7 +152,7 @@ def build_binding(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError(f"{cxx} linked libstdc++ statically into the torch binding; set FA8_CXX to a "
                                "g++ that links it dynamically")
     with open(out + ".srchash", "w") as f:
-        f.write(_binding_digest() + "\n")
+        f.write(_binding_digest() + " " + str(torch.__version__) + "\n")     # see binding_is_stale
     return out
 
 

@@ -38,3 +38,29 @@ def test_the_same_complaints_either_way(monkeypatch, native):
         api.flash_attention_v2_cutlass(q, q, q, False, 0.125, v_layout="upside down")
     with pytest.raises(RuntimeError, match="x must be a CUDA tensor"):
         api.quantize_e4m3(torch.zeros(4, 4, dtype=torch.float16))
+
+
+def test_a_module_built_for_another_torch_is_stale(monkeypatch):
+    build.build_binding()
+    monkeypatch.setattr(torch, "__version__", "1.0")
+    assert build.binding_is_stale()
+
+    def gone():
+        raise FileNotFoundError
+    monkeypatch.setattr(build, "_binding_digest", gone)          # an installed copy notices as well
+    assert build.binding_is_stale()
+
+
+@pytest.mark.parametrize("error", [ImportError("undefined symbol"), OSError("cannot open shared object file")])
+def test_a_module_that_does_not_load_leaves_ctypes(monkeypatch, error):
+    build.build_binding()
+
+    def broken(spec):
+        raise error
+    monkeypatch.setattr(api, "_native_module", None)
+    monkeypatch.setattr(api.importlib.util, "module_from_spec", broken)
+    with pytest.warns(UserWarning, match="through ctypes"):
+        assert api._native() is False
+    q = torch.zeros(1, 1, 128, 64).to(F8)
+    with pytest.raises(RuntimeError, match="q must be a CUDA tensor"):
+        api.flash_attention_v2_cutlass(q, q, q, False, 0.125, v_layout="natural")
