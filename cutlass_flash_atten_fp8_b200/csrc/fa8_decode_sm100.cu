@@ -15,8 +15,8 @@
 //     in which mma.m16n8k16 wants its operands (all loads are 8 or 16 bytes a thread, whole
 //     32-byte sectors), the next keys' loads in flight while the current ones are worked on.  There is no
 //     shared-memory staging, hence no barrier and no wait in the loop.  tcgen05 would want 128
-//     rows (or 128 lanes of keys and a transposed P through shared memory) for what is 24 small
-//     products per 8 KB read.
+//     rows (or 128 lanes of keys and a transposed P through shared memory) for what is 48 small
+//     products per 8 KB read (head dim 128, up to eight rows).
 //
 // Operand layouts.  S = Q K^T with the query rows as M (16, eight of them padding when RB = 1)
 // and eight keys as N; the k index of the instruction may be permuted as long as both operands
@@ -28,7 +28,10 @@
 //
 // Numerics are those of the prefill kernel: P = 2^(c s - c m) in fp32, rounded to fp8 after the
 // fp32 row sum, with m the exact row maximum over the first 64 keys of the slice (every warp of
-// the cluster starts from it), raised by a warp whose P of one step reaches beyond 448.
+// the cluster starts from it), raised by a warp, for itself, when the eight P of a thread in one step add
+// up to more than 448 (no single one is larger then).  How many CTAs and warps share the keys depends on the
+// number of slices and SMs, so the order of the fp32 sums, and which warps have raised their maximum, do
+// too: the last bits of a slice's output change with the other slices of the launch.
 #include <cooperative_groups.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -51,10 +54,9 @@ constexpr float kRaiseAbove = 448.f;   // largest e4m3 value
 
 // Every fp8 value is an fp16 value too, so a product of widened operands with an fp32 sum is the fp8
 // product.  The instruction's own fp8 form is carried out in fp16 as well on this architecture, but
-// widens both operands again for every product; widening each K and V word once by hand takes
-// about half as many
-// instructions (652 per warp step before, counted by ncu; 57 us before, 51 now at batch 16, 8 key/value
-// heads, 8192 keys, head dim 128).
+// widens both operands again for every product; widening each K and V word once by hand takes 421
+// instructions per warp step instead of 652 (ncu), 51 us instead of 57 at batch 16, 8 key/value heads,
+// 8192 keys, head dim 128.
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -541,12 +543,13 @@ int decode_split(int64_t items, int seqlen_k, int max_warps, int sms, int max_sp
   return best_split;
 }
 
-// Up to kDecodeRowsMax rows may come here.  A single block of rows always does: 5.2 TB/s of K and V
-// (78 % of a copy) against a step of 0.41 us per 64 keys (0.65 at head dim 256) and slice of the
-// prefill kernel.  Several blocks each read K and V (from L2, at the same rate per SM), so they
-// do when the prefill kernel would leave SMs idle - it does not split a slice's keys.  Measured,
-// head dim 128: 8 slices of 56 rows, 16384 keys of head dim 64: 18 us here, 105 there; 128 slices of
-// 48 rows, 4096 keys: 98 us here, 33 there.
+// Up to kDecodeRowsMax rows may come here.  A single block of rows always does.  Several blocks each
+// read K and V (from L2, at the same rate per SM), so they do when the prefill kernel would leave SMs
+// idle: it does not split a slice's keys.  Both sides' costs (us) are fits to launches of 4-160 slices of 16-56
+// rows, 1024 and 8192 keys; a head dim costs as much as the width of the instance it runs in (64 slices of 16
+// rows, 8192 keys, head dim 160 / 192 / 224: 103 / 106 / 109 us).  Measured, here against there: 16 slices of 56
+// rows, 8192 keys, head dim 64: 17, 61; 64 of them at 128: 98, 73; 32 slices of 16 rows, 8192 keys at 256:
+// 47, 70, 64 of them: 86, 71; of 1024 keys: 15.8, 14.8.
 bool decode_takes(int64_t slices, int64_t rows, int seqlen_k, int head_dim, int sms) {
   const int width = head_dim <= 64 ? 64 : (head_dim <= 128 ? 128 : 256);
   const int64_t block = width == 256 ? 8 : 16;
@@ -554,8 +557,9 @@ bool decode_takes(int64_t slices, int64_t rows, int seqlen_k, int head_dim, int 
   if (rows > kDecodeRowsMax || slices * row_blocks * 8 > 0x7fffffff) return false;
   if (row_blocks == 1) return true;
   const double keys = seqlen_k;
-  const double here = static_cast<double>(row_blocks) * slices * keys * 2.0 * width / 5.2e6;                  // us
-  const double there = static_cast<double>((slices + sms - 1) / sms) * (keys / 64.0 * (width == 256 ? 0.65 : 0.41) + 3.0);
+  const double step = width == 64 ? 0.43 : (width == 128 ? 0.51 : 0.49);                // of 64 keys there
+  const double here = static_cast<double>(row_blocks) * slices * keys * 2.0 * width / 4.7e6 + 3.0;
+  const double there = static_cast<double>((slices + sms - 1) / sms) * (keys / 64.0 * step + 5.5);
   return here < there;
 }
 
