@@ -4,12 +4,13 @@ the folding of query heads that share a key/value head into one slice.
 Against a model of it (the same rounding of P to fp8, starting maximum over the first 64 keys) the
 difference is the order of fp32 sums and, now and then, a P on the other side of a rounding step: 2e-3 as
 for the prefill kernel.  Against the fp32 oracle it is the rounding of P: 3e-2 (e5m2 6e-2)."""
+import ctypes
 import math
 
 import pytest
 import torch
 
-from cutlass_flash_atten_fp8_b200 import check_status, flash_attention_v2_cutlass
+from cutlass_flash_atten_fp8_b200 import _lib, check_status, flash_attention_v2_cutlass
 from oracle.attention_oracle import error_metrics
 
 pytestmark = pytest.mark.gpu
@@ -45,8 +46,15 @@ def rounded_p(q, k, v, scale, dtype):
     return p.to(dtype).float() @ v.float().repeat_interleave(g, 1) / p.sum(-1, keepdim=True)
 
 
+def taken(slices, rows, Sk, D):
+    """Whether the call goes to the decode kernel (fa8::decode_takes)."""
+    f = _lib.load()._ZN3fa812decode_takesElliii
+    f.restype, f.argtypes = ctypes.c_bool, [ctypes.c_int64, ctypes.c_int64] + 3 * [ctypes.c_int]
+    return f(slices, rows, Sk, D, torch.cuda.get_device_properties(0).multi_processor_count)
+
+
 # one key, less than the first 64, not a multiple of a 32-key step, one step more than a split of two to
-# eight CTAs of four warps; 1, 7, 8, 9, 16, 17, 64 and 65 rows (the last one past the decode kernel)
+# eight CTAs of four warps; 1, 2, 7, 8, 9, 16 and 17 rows; 64 and 65 (past the decode kernel: folded prefill)
 @pytest.mark.parametrize("H,Hk,Sq,Sk,D", [
     (2, 2, 1, 1, 32), (2, 1, 1, 33, 64), (4, 2, 1, 64, 128), (7, 1, 1, 65, 128), (8, 1, 1, 1000, 256), (3, 1, 3, 777, 96),
     (2, 1, 8, 4097, 64), (17, 1, 1, 2049, 160), (16, 2, 8, 1056, 128), (5, 1, 13, 513, 192), (8, 1, 2, 288, 224)])
@@ -106,3 +114,37 @@ def test_an_infinite_value_of_the_last_key_comes_through(D, col, Sk):
     assert float(out[0, 0, 0, col]) == math.inf
     plain[0, 0, 0, col] = math.inf
     assert torch.equal(out, plain)
+
+
+# blocks of rows: one more row than fits a block, the last block full or of one row, at either end of the kernels'
+# head dims; the most rows there are, and one more.  A row's output is rounded to fp16 (2^-11) after sums in another
+# order: 1e-3.  The kernel's fp32 exponentials are off by about 3e-7 of their value and roundings lie 2^-4 to 2^-3 of it
+# apart (e5m2 2^-3 to 2^-2), so of the 1e5 to 3e5 probabilities of a case one or two may be rounded the other way: such a row
+# is off by a step of its largest P (at most 2^-3, e5m2 2^-2, of it) times that key's value.
+@pytest.mark.parametrize("rows,group", [(17, 17), (32, 4), (33, 3), (48, 6), (63, 7)])
+@pytest.mark.parametrize("D", [32, 64, 96, 128, 160, 256])
+def test_several_row_blocks(rows, group, D):
+    Hk, Sk = (1, 1500) if D % 64 else (2, 2049)
+    assert taken(2 * Hk, rows, Sk, D) and not taken(2 * Hk, 64, Sk, D)
+    dtype = torch.float8_e5m2 if rows == 33 else torch.float8_e4m3fn
+    q, k, v = (rand8(2, h, s, D, seed=Sk + i, dtype=dtype) for i, (h, s) in enumerate([(group * Hk, rows // group), (Hk, Sk), (Hk, Sk)]))
+    scale = 1 / math.sqrt(D)
+    out, lse = call(q, k, v, scale)
+    want = rounded_p(q, k, v, scale, dtype)
+    ref, ref_lse = reference(q, k, v, scale)
+    off, size = (out - want).norm(dim=-1), want.norm(dim=-1)
+    # P relative to the row sum: exp(largest score - log-sum-exp)
+    s = q.float() @ k.float().repeat_interleave(group, 1).transpose(2, 3) * scale
+    step = (0.25 if rows == 33 else 0.125) * torch.exp(s.amax(-1) - ref_lse) * v.float().norm(dim=-1).max()
+    turned = off > 1e-3 * size
+    assert int(turned.sum()) <= 2
+    assert bool((off <= 1e-3 * size + 2 * step * turned).all())
+    assert float((lse - ref_lse).abs().max()) <= 1e-5 * float(ref_lse.abs().max()) + 1e-5
+
+
+@pytest.mark.parametrize("rows,Sk", [(18, 2000), (63, 1300), (195, 300), (390, 500)])
+def test_scales_per_head_over_row_blocks_and_folded_tiles(rows, Sk):
+    Sq = rows // 3                                   # groups of three heads: heads share a block of rows or a tile
+    assert taken(4, rows, Sk, 64) == (rows < 64)
+    assert rows < 64 or (rows + 127) // 128 < 3 * ((Sq + 127) // 128)          # folded
+    test_scales_per_head_follow_the_heads_of_a_group(Sq, Sk)
