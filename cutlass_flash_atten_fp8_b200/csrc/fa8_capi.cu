@@ -141,10 +141,11 @@ DeviceState* device_state() {
   return &st;
 }
 
-// Scratch of fa8_quantize_e4m3_segments_noalloc: the per-segment |x| maxima that the first pass
-// accumulates and the second pass reads.  A file-scope device array instead of memory from the
-// allocator: 16 KB on every GPU that loads the library, held until the process exits, shared by
-// every call (so it keeps the last call's contents and is cleared at the start of each).
+// Scratch of fa8_quantize_e4m3_segments_noalloc: the per-segment |x| maxima (of two passes the
+// first accumulates and the second reads them; a cluster per segment only writes them).  A
+// file-scope device array instead of memory from the allocator: 16 KB on every GPU that loads the
+// library, held until the process exits, shared by every call (so it keeps the last call's
+// contents; a call writes an entry before it reads it).
 static __device__ __align__(256) float g_quant_amax_scratch[FA8_NOALLOC_MAX_SEGMENTS];
 
 // In host code the array's name is only a handle for the runtime, not an address a kernel can
@@ -444,8 +445,8 @@ int fa8_quantize_e4m3_segments_noalloc(const void* src, int32_t src_dtype, void*
     set_detail("cudaGetSymbolAddress (quantiser scratch)", cudaGetErrorString(e));
     return FA8_ERR_CUDA;
   }
-  // launch_quantize clears the n_seg maxima it is about to accumulate (stream-ordered), runs the
-  // two passes and allocates nothing.
+  // launch_quantize writes the n_seg maxima before it reads them (stream-ordered) and allocates
+  // nothing.
   e = fa8::launch_quantize(src, src_dtype == FA8_DTYPE_BF16, dst, seg_len, n_seg, amax, descale,
                            static_cast<cudaStream_t>(cuda_stream));
   if (e != cudaSuccess) {

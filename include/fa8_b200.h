@@ -183,10 +183,13 @@ int fa8_supported(int32_t seqlen_k, int32_t head_dim, int32_t v_layout);
  * items of 256 query rows (two 128-row tiles side by side; one tile at head dims above 128);
  * a causal unit pairs item f with item n-1-f of a slice so that all units cost the same.
  * Problems that would leave more than half of the SMs idle are cut finer: items of 128 rows,
- * or causal items as units of their own.  Results do not depend on the plan.  (Launches without a
+ * or causal items as units of their own.  Results do not depend on the plan, nor a slice's on the other
+ * slices of the launch.  (Launches without a
  * causal mask whose query heads share key/value heads are first regrouped, slices = batch *
- * heads_kv of heads / heads_kv * seqlen rows, where that needs fewer 128-row tiles; those of fewer than
- * 64 such rows with natural V may go to the decode kernel, which splits the keys instead.)
+ * heads_kv of heads / heads_kv * seqlen rows, where that needs fewer 128-row tiles.  Those of fewer than
+ * 64 such rows with natural V may go to the decode kernel, which has no such plan: it splits a slice's
+ * keys by the number of slices and SMs, so there a slice's result varies with them, by the order of
+ * fp32 sums and, where a row maximum is raised on the way, by roundings of the fp8 probabilities.)
  * plan[0] = query rows per item, plan[1] = 1 if causal items are paired, plan[2] = items per
  * slice, plan[3] = units (the grid is min(units, sm_count) CTAs).  seqlen_k 0 = seqlen. */
 int fa8_work_plan(int32_t slices, int32_t seqlen, int32_t seqlen_k, int32_t head_dim, int32_t is_causal,
